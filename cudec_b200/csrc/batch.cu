@@ -34,6 +34,13 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::atomic<int> g_sm_count[kMaxDevices];
 
+// Chunks per SM up to which a batch's chunks get 512 or 256 threads each. Us
+// per batch of 64 KiB LZ4 chunks with 512 / 256 / 128 threads on 148 SMs: 148
+// chunks 174 / 201 / 300, 300 chunks 330 / 216 / 312, 440 chunks 387 / 234 /
+// 337, 592 chunks 527 / 393 / 357, 1,024 chunks 856 / 563 / 447; 16 chunks of
+// 4 MiB 9,550 / 11,720 / 15,980.
+constexpr size_t kWideMax = 1, kMediumMax = 3;
+
 }  // namespace
 
 int device_sm_count(int dev) {
@@ -46,51 +53,59 @@ int device_sm_count(int dev) {
     return v;
 }
 
-// The CTA-per-chunk kernel's resident CTAs per SM, once per device and
-// format (its shared state exceeds 48 KB: opted into here).
-template <class F>
-cudaError_t prepare_cta(std::atomic<int>* ready, int dev, int* per_sm) {
+// The kernel's shared state exceeds 48 KB: opted into once per device, format
+// and width.
+template <class F, uint32_t T>
+cudaError_t prepare_cta(int dev) {
+    static std::atomic<bool> ready[kMaxDevices];
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-    int v = ready[dev].load(std::memory_order_acquire);
-    if (v > 0) {
-        *per_sm = v;
-        return cudaSuccess;
-    }
-    constexpr int kSmem = static_cast<int>(sizeof(lzc::Shm<F>));
-    cudaError_t e = cudaFuncSetAttribute(lzc::lz_cta_kernel<F>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, lzc::lz_cta_kernel<F>, lzc::kThreads,
-                                                      kSmem);
-    if (e != cudaSuccess) return e;
-    if (v <= 0) return cudaErrorInvalidConfiguration;
-    ready[dev].store(v, std::memory_order_release);
-    *per_sm = v;
-    return cudaSuccess;
+    if (ready[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(lzc::lz_cta_kernel<F, T>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(sizeof(lzc::Shm<F, T>)));
+    if (e == cudaSuccess) ready[dev].store(true, std::memory_order_release);
+    return e;
 }
 
-std::atomic<int> g_lz4_cta_ready[kMaxDevices];
-std::atomic<int> g_snappy_cta_ready[kMaxDevices];
+struct Batch {
+    const void* const* src;
+    const size_t* src_sizes;
+    void* const* dst;
+    const size_t* caps;
+    size_t n;
+    cudec_chunk_result* results;
+    cudaStream_t stream;
+    int dev;
+};
 
-// One CTA per chunk at a time, persistent over the batch.
+// One CTA of T threads per chunk (the hardware hands CTAs out as SMs fall
+// free, so uneven chunks balance).
+template <class F, uint32_t T>
+cudec_status launch_width(const Batch& b) {
+    if (prepare_cta<F, T>(b.dev) != cudaSuccess) return CUDEC_ERR_CUDA;
+    constexpr size_t kMaxGrid = INT32_MAX;
+    const unsigned grid = static_cast<unsigned>(b.n < kMaxGrid ? b.n : kMaxGrid);
+    lzc::lz_cta_kernel<F, T><<<grid, T, sizeof(lzc::Shm<F, T>), b.stream>>>(
+        b.src, b.src_sizes, b.dst, b.caps, b.n, b.results);
+    return cudaGetLastError() == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
+}
+
 template <class F>
-static cudec_status launch_lz_cta(std::atomic<int>* ready, const void* const* src,
-                                  const size_t* src_sizes, void* const* dst, const size_t* caps,
-                                  size_t n, cudec_chunk_result* results, cudaStream_t stream) {
+cudec_status launch_lz_cta(const void* const* src, const size_t* src_sizes, void* const* dst,
+                           const size_t* caps, size_t n, cudec_chunk_result* results,
+                           cudaStream_t stream) {
     const cudec_status v = validate_batch(src, src_sizes, dst, caps, n, results);
     if (v != CUDEC_OK) return v;
     (void)cudaGetLastError();
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return CUDEC_ERR_CUDA;
-    int per_sm = 0;
-    if (prepare_cta<F>(ready, dev, &per_sm) != cudaSuccess) return CUDEC_ERR_CUDA;
-    const int sms = device_sm_count(dev);
-    if (sms <= 0) return CUDEC_ERR_CUDA;
-    const size_t max_blocks = static_cast<size_t>(sms) * per_sm;
-    const unsigned grid = static_cast<unsigned>(n < max_blocks ? n : max_blocks);
-    lzc::lz_cta_kernel<F><<<grid, lzc::kThreads, sizeof(lzc::Shm<F>), stream>>>(
-        src, src_sizes, dst, caps, n, results);
-    return cudaGetLastError() == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
+    Batch b{src, src_sizes, dst, caps, n, results, stream, 0};
+    if (cudaGetDevice(&b.dev) != cudaSuccess) return CUDEC_ERR_CUDA;
+    const size_t sms = static_cast<size_t>(device_sm_count(b.dev));
+    if (sms == 0) return CUDEC_ERR_CUDA;
+    // A wide CTA shortens a chunk's own time, narrow ones use the SM better:
+    // wide while the batch leaves SMs idle otherwise.
+    if (n <= kWideMax * sms) return launch_width<F, 512>(b);
+    if (n <= kMediumMax * sms) return launch_width<F, 256>(b);
+    return launch_width<F, 128>(b);
 }
 
 }  // namespace cdb
@@ -105,7 +120,7 @@ cudec_status cudec_lz4_decompress_batch(const void* const* d_src_ptrs,
                                         cudec_chunk_result* d_results,
                                         cudec_stream_t stream) {
     return cdb::launch_lz_cta<cdb::lzc::Lz4F>(
-        cdb::g_lz4_cta_ready, d_src_ptrs, d_src_sizes, d_dst_ptrs, d_dst_capacities,
+        d_src_ptrs, d_src_sizes, d_dst_ptrs, d_dst_capacities,
         chunk_count, d_results, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -117,7 +132,7 @@ cudec_status cudec_snappy_decompress_batch(const void* const* d_src_ptrs,
                                            cudec_chunk_result* d_results,
                                            cudec_stream_t stream) {
     return cdb::launch_lz_cta<cdb::lzc::SnappyF>(
-        cdb::g_snappy_cta_ready, d_src_ptrs, d_src_sizes, d_dst_ptrs,
+        d_src_ptrs, d_src_sizes, d_dst_ptrs,
         d_dst_capacities, chunk_count, d_results,
         reinterpret_cast<cudaStream_t>(stream));
 }

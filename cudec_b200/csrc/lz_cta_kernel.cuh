@@ -1,48 +1,58 @@
 // CTA-per-chunk decoder for the byte-oriented LZ formats (LZ4 block, raw
-// Snappy): the chunk's token chain is found in parallel by the whole CTA,
-// and the tokens execute one per thread.
+// Snappy): the chunk's token chain is found by every thread of the CTA
+// walking a stretch of the input speculatively, tokens are parsed one per
+// thread, and the output is produced one byte per lane by gathering.
 //
 // A chunk is decoded tile by tile. A tile is the kTile input positions that
-// start at a known token (the chunk's first, then each tile's exit). For a
-// tile, with kThreads threads:
+// start at a known token (the chunk's first, then each tile's exit):
 //
 //   1. stage: the tile's input bytes (plus kLook bytes past it) land in
-//      shared memory by cp.async, in aligned 16-byte blocks;
-//   2. segment exits: thread t owns the kSeg positions of segment t and,
-//      walking them backwards, computes for every position p the exit of
-//      the chain that starts at p: the first chain position at or past the
-//      segment's end (the format's step, its length extensions capped at
-//      kExtCap bytes; a position the cap stops is "unknown");
-//   3. candidate chase: warp w owns super-segment w (kSupSegs segments) and
-//      lane k follows the chain from the super-segment's k-th position
-//      through its segments by their exits, recording where it enters each
-//      segment; the true entry into a super-segment lies within its first
-//      kCand positions unless a token straddles its start by more;
-//   4. tile chase: one thread follows the true chain through the tile's
-//      super-segments, picking the lane whose start is the true entry (an
-//      unknown exit, or an entry past the candidates, is resolved by
-//      walking that super-segment exactly);
-//   5. count: each thread walks its segment from its true entry (exact
-//      steps), counting tokens and output bytes; a block scan gives every
-//      token its index and output offset;
-//   6. check: each thread walks its segment again and runs the format's
-//      exact ladder (lz_ladder.cuh) on each token at its output offset; the
-//      first failing or terminal token (a block-wide minimum) decides the
-//      chunk exactly as the serial parser would, since the steps equal the
-//      ladder's next position for every token the ladder accepts;
-//   7. execute, in groups of consecutive tokens whose output fits kGroupOut:
-//      the group's literal runs are copied into an output ring in shared
-//      memory (indexed by destination address mod kRing, so ring blocks and
-//      destination blocks share alignment), then its matches as data flow:
-//      each thread copies each of its matches once none of the bytes its
-//      source reads is the output of a match still pending in the group (a
-//      bit per output byte), and clears the match's own bits after its bytes
-//      land; the lowest pending match is always ready, so the group always
-//      makes progress.
-//      Completed aligned 16-byte blocks leave the ring as coalesced stores.
-//      A token longer than kBig is copied by the whole CTA straight to the
-//      destination. Sources older than the ring are read back from the
-//      destination.
+//      shared memory by cp.async, in aligned 16-byte blocks, while the tile
+//      before runs;
+//   2. steps and exits: the distance to the next token from every position
+//      (the format's step, without branches, four positions at a time), and
+//      from every position of a region (kReg positions, one region per
+//      thread) the distance to the first chain position past the region,
+//      computed backwards;
+//   3. settle: region t is entered at region t - 1's exit. Every region
+//      starts from the exit of its first position; LZ chains started
+//      anywhere merge after a few tokens, so most are right at once. In a
+//      round, the first region f whose entry is not its neighbour's exit
+//      takes it (everything before f is right), a region that the chain
+//      leaving f - 1 passes over takes that exit too, and any other region
+//      takes its neighbour's exit where that lies inside it; each looks its
+//      own exit up. Only region f takes an uncommon step (a long extension,
+//      the chunk's end), the others leave it open, to be taken when they are
+//      first. Rounds repeat until every region is settled; after kRounds of
+//      them (content with few tokens per region) one thread follows the
+//      chain through the rest, a look-up per region;
+//   4. list: each thread walks its region from its entry; a scan of the
+//      counts gives every token its index, and the tokens' positions go to a
+//      list;
+//   5. batches of kThreads tokens, one per thread: parse (the format's fast
+//      form, the exact ladder of lz_ladder.cuh where it declines), a scan of
+//      the output lengths, the ladder's conditions at the token's output
+//      offset (the first failing or terminal token decides the chunk as the
+//      serial parser would, since the steps equal the ladder's next position
+//      for every token the ladder accepts), and a map of the batch's output:
+//      one start bit per output byte and the token count before each aligned
+//      32-byte sector;
+//   6. copy: a warp writes whole 32-byte sectors of the destination, one
+//      byte per lane. A byte's token is the sector's count plus a popcount
+//      of the start bits up to it; a literal byte comes from the staged
+//      input, a match byte from the destination. A match byte whose source
+//      lies in the same window is followed through the map (a period is
+//      taken modulo its length, so a match costs one hop) until a literal
+//      or a byte before the window is met, so no byte waits for another.
+//      A token longer than kBig is copied by the whole CTA, 16 bytes per
+//      thread at a time.
+//
+// What bounds it: instruction issue (77 % of the issue slots at seven CTAs per
+// SM; 290,000 warp instructions per 64 KiB chunk of 5,250 tokens, two thirds
+// of them in the copy). The decoder before this one computed chain exits by
+// the format's branching step, merged 16-byte pieces per token into a
+// shared-memory ring with atomics, and spent 568,000. 1,024 chunks of 64 KiB
+// on a B200: LZ4 0.943 -> 0.437 ms (154 GB/s out), Snappy 1.149 -> 0.457.
 //
 // Every phase is per-thread code between CTA barriers, driven through an
 // executor: on the device each phase runs once per thread followed by
@@ -59,79 +69,71 @@
 #include <cstring>
 
 #include "cudec.h"
+#include "lz_gather.cuh"
 #include "lz_ladder.cuh"
 
 namespace cdb {
 namespace lzc {
 
-constexpr uint32_t kThreads = 256;                 // threads per CTA
-constexpr uint32_t kCtasPerSm = 4;                 // resident CTAs per SM the registers allow
-constexpr uint32_t kWarps = kThreads / 32;
-constexpr uint32_t kSeg = 16;                      // positions per segment (one per thread)
-constexpr uint32_t kTile = kThreads * kSeg;        // positions per tile
-constexpr uint32_t kSupSegs = 32;                  // segments per super-segment (a warp)
-constexpr uint32_t kSupers = kThreads / kSupSegs;  // super-segments per tile
-constexpr uint32_t kSupPos = kSupSegs * kSeg;
-constexpr uint32_t kCand = 32;                     // candidate entries per super-segment
-constexpr uint32_t kLook = 512;                    // staged bytes past the tile
-constexpr uint32_t kInBytes = kTile + kLook + 32;  // staged input (aligned blocks)
-constexpr uint32_t kExIdx = kTile + kTile / 16;    // exits, one pad word per 16
-constexpr uint32_t kRing = 16384;                  // output ring (bytes)
-constexpr uint32_t kGroupOut = 4096;               // output bytes per execution group
-constexpr uint32_t kPerThread = 2;                 // tokens per thread per group
-constexpr uint32_t kGroupTok = kThreads * kPerThread;
-constexpr uint32_t kBig = 256;                     // longer tokens: whole-CTA copies
-constexpr uint32_t kExtCap = 16;                   // extension bytes a segment step reads
-constexpr uint32_t kSpinCap = 1u << 22;            // passes a thread makes over its matches
+constexpr uint32_t kThreads = 128;  // threads per CTA unless a chunk gets more
+constexpr uint32_t kReg = 52;       // positions per region: at most 64 (a mask), an odd number of
+                                    // words (no bank conflicts where the regions are walked)
+constexpr uint32_t kLook = 512;     // staged bytes past the tile
+using lzg::kSectors;
+using lzg::kWindow;
+using lzg::Rec;
+using lzg::Sector;
+constexpr uint32_t kBig = 1024;                    // longer tokens: whole-CTA copies
+constexpr uint32_t kExtCap = 16;                   // extension bytes a fast parse reads
 
-static_assert(kSupers == kWarps, "one super-segment per warp");
-static_assert(kGroupOut + 32 <= kRing, "a group and its clear margin fit the ring");
-static_assert(kInBytes % 16 == 0, "staging in 16-byte blocks");
+// What follows from the CTA's width.
+template <uint32_t T>
+struct Width {
+    static constexpr uint32_t kWarps = T / 32;
+    static constexpr uint32_t kTile = T * kReg;  // positions per tile: a region per thread
+    static constexpr uint32_t kInBytes = (kTile + kLook + 32 + 15) / 16 * 16;  // staged input
+    static constexpr uint32_t kUnroll = T == 128 ? 4 : 2;      // sectors in flight per warp
+    static constexpr uint32_t kPart = 32 * kWarps * kUnroll;  // output bytes between barriers
+    // resident CTAs per SM that the registers are compiled for
+    static constexpr int kPerSm = T == 128 ? 7 : T == 256 ? 3 : 1;
+};
 
-// Exit codes of the segment walk (relative positions otherwise).
-constexpr uint32_t kUnknown = 0xFFFFFFFFu;  // a step the cap stopped: resolve exactly
-constexpr uint32_t kEndMark = 0xFFFFFFFEu;  // the chain ends inside this segment
-constexpr uint32_t kFarRel = 0xFFFFFFF0u;   // relative positions at or above: unknown
+static_assert(kReg <= 64 && kReg % 8 == 4, "a region's mask is one word; odd in 4-byte words");
+
+// Region exits: positions relative to the tile's entry, or
+constexpr uint32_t kExitEnd = 0xFFFFFFFFu;   // the chain ends (its last token is noted)
+constexpr uint32_t kExitFar = 0xFFFFFFFEu;   // 2^31 or further: s.far
+constexpr uint32_t kExitOpen = 0xFFFFFFFDu;  // a step left open: not known to be on the chain
+constexpr uint32_t kExitMax = 0x80000000u;   // positions are below this
 
 // Step results (absolute positions otherwise).
-constexpr uint64_t kStepUnknown = ~0ull;
-constexpr uint64_t kStepEnd = ~0ull - 1;
+constexpr uint64_t kStepEnd = ~0ull;
 constexpr uint32_t kSlowRel = 0xFFFFFFFFu;  // a fast step declines: the generic step decides
-
-// Entry codes of the candidate chase (offsets into a segment otherwise).
-constexpr uint8_t kNoEntry = 0xFF;   // no chain token starts in the segment
-constexpr uint8_t kCodeUnk = 0xFE;   // the chain became unknown before the segment
-constexpr uint8_t kCodeEnd = 0xFD;   // the chain ended before the segment
-constexpr uint8_t kChoseOvr = 0xFC;  // super-segment resolved by an exact walk
-
-// The tile's first event (first failing or terminal token).
-constexpr uint8_t kEvNone = 0;
-constexpr uint8_t kEvDone = 1;  // terminal token accepted: the chunk ends after it
-constexpr uint8_t kEvFail = 2;  // rejected: ev_status holds the status
+constexpr uint32_t kStepSlow = 255;         // no short step from this position
+constexpr uint32_t kRounds = 12;            // settling rounds before the serial finish
 
 // ---------------------------------------------------------------------------
 // Portable primitives (device: the real thing; host: the sequential
 // emulation's plain operations).
-#if defined(__CUDA_ARCH__)
+#if CDB_DEVICE_CODE
 #define LZC_LDG(p) __ldg(p)
-__device__ __forceinline__ void at_or(uint32_t* a, uint32_t v) { atomicOr(a, v); }
-__device__ __forceinline__ void at_and(uint32_t* a, uint32_t v) { atomicAnd(a, v); }
 __device__ __forceinline__ void at_min(uint32_t* a, uint32_t v) { atomicMin(a, v); }
+__device__ __forceinline__ uint32_t pop64(uint64_t v) { return __popcll(v); }
+__device__ __forceinline__ uint32_t ctz64(uint64_t v) { return __ffsll(v) - 1; }
 #else
 #define LZC_LDG(p) (*(p))
-inline void at_or(uint32_t* a, uint32_t v) { *a |= v; }
-inline void at_and(uint32_t* a, uint32_t v) { *a &= v; }
 inline void at_min(uint32_t* a, uint32_t v) {
     if (v < *a) *a = v;
 }
+inline uint32_t pop64(uint64_t v) { return static_cast<uint32_t>(__builtin_popcountll(v)); }
+inline uint32_t ctz64(uint64_t v) { return static_cast<uint32_t>(__builtin_ctzll(v)); }
 #endif
 
 // Profiling builds (-DCDB_PHASE_TIMING) accumulate, from thread 0 of every
 // CTA, the SM cycles of each phase and event counts over a launch. Cycles:
-// 0 stage, 1 segment exits, 2 candidate chase, 3 tile chase, 4 count and
-// scan, 5 check, 6 group clear and literals, 7 match rounds, 8 flush,
-// 9 whole-CTA tokens, 10 group cut. Events: 0 tiles, 1 tokens, 2 rounds,
-// 3 groups, 4 whole-CTA tokens, 5 exact walks.
+// 0 stage, 1 steps, 2 exits and settle, 3 list, 4 parse and scan, 5 check and map,
+// 6 copy, 7 whole-CTA tokens. Events: 0 tiles, 1 tokens, 2 settle rounds,
+// 3 batches, 4 whole-CTA tokens, 5 windows.
 #if defined(CDB_PHASE_TIMING) && defined(__CUDACC__)
 __device__ unsigned long long lzc_cycles[16];
 __device__ unsigned long long lzc_events[16];
@@ -162,27 +164,13 @@ __device__ unsigned long long lzc_events[16];
     } while (0)
 #endif
 
-CDB_HD uint32_t fsr(uint32_t lo, uint32_t hi, uint32_t sh) {  // funnel shift right, sh < 32
-    return sh ? (lo >> sh) | (hi << (32 - sh)) : lo;
-}
-CDB_HD uint32_t fsl(uint32_t lo, uint32_t hi, uint32_t sh) {  // (hi:lo) << sh, high word
-    return sh ? (hi << sh) | (lo >> (32 - sh)) : hi;
-}
-CDB_HD uint32_t keep_low(uint32_t w, uint32_t bits) {  // low `bits` (0..32) bits of w
-    return bits >= 32 ? w : (w & ((1u << bits) - 1u));
-}
-
-struct V16 {
-    uint32_t w[4];
-};
-
 // ---------------------------------------------------------------------------
 // Phases. each(fn): fn(tid) for every thread of the CTA, then a barrier (on
-// the host: every thread in turn). each_or: the same, and whether any call
-// returned true. The host forms emulate the CTA sequentially.
-template <class Fn>
+// the host: every thread in turn). The host forms emulate the CTA
+// sequentially.
+template <uint32_t kThreads, class Fn>
 CDB_HD void each(Fn fn) {
-#if defined(__CUDA_ARCH__)
+#if CDB_DEVICE_CODE
     fn(threadIdx.x);
     __syncthreads();
 #else
@@ -190,16 +178,43 @@ CDB_HD void each(Fn fn) {
 #endif
 }
 
-template <class Fn>
-CDB_HD bool each_or(Fn fn) {
-#if defined(__CUDA_ARCH__)
-    return __syncthreads_or(fn(threadIdx.x)) != 0;
+// The same without the barrier.
+template <uint32_t kThreads, class Fn>
+CDB_HD void each_free(Fn fn) {
+#if CDB_DEVICE_CODE
+    fn(threadIdx.x);
 #else
-    bool any = false;
-    for (uint32_t t = 0; t < kThreads; ++t) any = fn(t) || any;
-    return any;
+    for (uint32_t t = 0; t < kThreads; ++t) fn(t);
 #endif
 }
+
+// each(), with the threads whose call returned true as a bit each in words.
+template <uint32_t kThreads, class Fn>
+CDB_HD void vote(uint32_t* words, Fn fn) {
+#if CDB_DEVICE_CODE
+    const uint32_t b = __ballot_sync(0xffffffffu, fn(threadIdx.x));
+    if ((threadIdx.x & 31) == 0) words[threadIdx.x >> 5] = b;
+    __syncthreads();
+#else
+    for (uint32_t t = 0; t < kThreads; ++t) {
+        if (t % 32 == 0) words[t / 32] = 0;
+        if (fn(t)) words[t / 32] |= 1u << (t % 32);
+    }
+#endif
+}
+
+// A value that each thread keeps from phase to phase: a register on the
+// device, one slot per thread on the host.
+template <class V, uint32_t kThreads>
+struct Priv {
+#if CDB_DEVICE_CODE
+    V v;
+    __device__ __forceinline__ V& operator[](uint32_t) { return v; }
+#else
+    V v[kThreads];
+    V& operator[](uint32_t t) { return v[t]; }
+#endif
+};
 
 // 16 bytes global -> shared (an aligned block); completed by land().
 CDB_HD void copy16_async(uint8_t* d, const uint8_t* src) {
@@ -217,58 +232,45 @@ CDB_HD void land_async() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_all;" ::: "memory");
 #endif
 }
-CDB_HD void st16(uint8_t* d, const uint8_t* src) {  // both 16-byte aligned
-#if defined(__CUDA_ARCH__)
-    *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(src);
-#else
-    std::memcpy(d, src, 16);
-#endif
-}
-CDB_HD void zero16(uint8_t* p) {  // 16-byte aligned
-#if defined(__CUDA_ARCH__)
-    *reinterpret_cast<uint4*>(p) = make_uint4(0, 0, 0, 0);
-#else
-    std::memset(p, 0, 16);
-#endif
-}
-
-// The first m (1..16) bytes of v at global address p.
-CDB_HD void put_global(uint8_t* p, const V16& v, uint32_t m) {
-#if defined(__CUDA_ARCH__)
-    if (m == 16 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        *reinterpret_cast<uint4*>(p) = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]);
-        return;
-    }
-    for (uint32_t j = 0; j < m; ++j) p[j] = static_cast<uint8_t>(v.w[j >> 2] >> (8 * (j & 3)));
-#else
-    std::memcpy(p, v.w, m);
-#endif
-}
-
 // ---------------------------------------------------------------------------
-// Formats: the exact ladder plus the segment step.
+// Formats: the exact ladder plus the step of the walk and the fast parse.
+
+// The staged bytes by position relative to the tile's entry.
+struct Staged {
+    const uint8_t* in;  // the staging buffer, 16-byte aligned
+    uint32_t at0;       // the entry's index in it
+    CDB_HD uint32_t at(uint32_t r) const { return in[at0 + r]; }
+    CDB_HD uint32_t word(uint32_t r) const {  // the four bytes from r
+        const uint32_t i = at0 + r;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(in) + (i >> 2);
+        return lzg::fsr(w[0], w[1], 8 * (i & 3));
+    }
+};
+
+// A token's fields as the fast parse reads them; positions relative to the
+// tile's entry.
+struct Tok {
+    uint32_t lit, ml, off;
+    uint32_t ls;  // position of the literal run
+};
 
 // LZ4: next = the ladder's next position for every token it accepts as
 // non-terminal; kStepEnd when the token can have no successor (the ladder
-// then answers terminal or reject); kStepUnknown when an extension run is
-// longer than `cap` bytes (cap 0: no limit).
+// then answers terminal or reject).
 struct Lz4F : lzl::Lz4Ladder {
-    static constexpr uint32_t kMaxTok = kTile / 3 + 3;  // tokens with a successor span >= 3 bytes
+    static constexpr uint32_t kMinStep = 3;  // tokens with a successor span >= 3 bytes
     static constexpr bool kSnappy = false;
 
     template <class R>
-    CDB_HD static uint64_t step(const R& in, uint64_t S, uint64_t P, uint32_t cap,
-                                uint64_t* olen) {
+    CDB_HD static uint64_t step(const R& in, uint64_t S, uint64_t P, uint64_t* olen) {
         if (P >= S) return kStepEnd;
         const uint32_t tok = in.at(P);
         uint64_t q = P + 1;
         uint64_t lit = tok >> 4;
         uint32_t b;
         if (lit == 15) {
-            uint32_t k = 0;
             do {
                 if (q >= S) return kStepEnd;
-                if (cap && k++ == cap) return kStepUnknown;
                 b = in.at(q++);
                 lit += b;
             } while (b == 255);
@@ -278,10 +280,8 @@ struct Lz4F : lzl::Lz4Ladder {
         q += lit + 2;
         uint64_t ml = (tok & 15) + 4;
         if ((tok & 15) == 15) {
-            uint32_t k = 0;
             do {
                 if (q >= S) return kStepEnd;
-                if (cap && k++ == cap) return kStepUnknown;
                 b = in.at(q++);
                 ml += b;
             } while (b == 255);
@@ -289,79 +289,115 @@ struct Lz4F : lzl::Lz4Ladder {
         *olen = lit + ml;
         return q;
     }
-    // Position of the literal run of the token at P with lit literal bytes.
-    template <class R>
-    CDB_HD static uint64_t lit_src(const R&, uint64_t P, uint64_t lit) {
-        return P + 1 + (lit >= 15 ? (lit - 15) / 255 + 1 : 0);
-    }
 
-    // Fast forms over the staged bytes, for a token whose header (with at
-    // most kExtCap extension bytes per length) lies well inside them and well
-    // before the chunk's end: b[r] is the token, lim = min(staged bytes, S)
-    // relative to b. kSlowRel: the generic forms decide.
+    // The step over the staged bytes without branches, for a token whose
+    // header (with at most one extension byte per length, below 255) lies
+    // well inside them and well before the chunk's end: word(in, r) are the
+    // four bytes from position r, lim = min(staged bytes, rest), rest = bytes
+    // to the chunk's end. kSlowRel: the other forms decide.
     static constexpr uint32_t kMargin = 2 * kExtCap + 2 + kSrcSlack;
-    CDB_HD static uint32_t ext_rel(const uint8_t* b, uint32_t* q, uint32_t* len) {
-        for (uint32_t k = 0; k < kExtCap; ++k) {
-            const uint32_t x = b[(*q)++];
-            *len += x;
-            if (x != 255) return 1;
-        }
-        return 0;
-    }
-    CDB_HD static uint32_t step_rel(const uint8_t* b, uint32_t r, uint32_t lim,
-                                    uint32_t* olen) {
+    CDB_HD static uint32_t hop_rel(const Staged& in, uint32_t r, uint32_t lim, uint32_t) {
         if (r + kMargin > lim) return kSlowRel;
-        const uint32_t tok = b[r];
-        uint32_t q = r + 1, lit = tok >> 4;
-        if (lit == 15 && !ext_rel(b, &q, &lit)) return kSlowRel;
+        const uint32_t u = in.word(r);
+        uint32_t lit = (u >> 4) & 15;
+        const uint32_t x1 = (u >> 8) & 255, e = lit == 15;
+        lit += e ? x1 : 0;
+        const uint32_t q = r + 1 + e + lit;  // the offset's position
+        if (q + 2 + kExtCap + kSrcSlack > lim) return kSlowRel;
+        const bool m = (u & 15) == 15;
+        const bool far = (e && x1 == 255) || (m && in.at(q + 2) == 255);
+        return far ? kSlowRel : q + 2 + m;
+    }
+    // hop_rel's distances from positions r..r+3 (r a multiple of 4), a byte
+    // each, all four at once; kStepSlow where it declines or the distance is
+    // longer than 146.
+    CDB_HD static uint32_t steps_rel(const Staged& in, uint32_t r, uint32_t lim) {
+        if (r + 3 + 160 + kMargin > lim) return steps_end(in, r, lim);
+        const uint32_t u = in.word(r), x1 = lzg::fsr(u, in.word(r + 4), 8);
+        constexpr uint32_t k1 = 0x01010101u;
+        const uint32_t lit = (u >> 4) & 0x0f0f0f0fu;
+        const uint32_t e = ((lit + k1) >> 4) & k1;                // an extended literal length
+        const uint32_t m = (((u & 0x0f0f0f0fu) + k1) >> 4) & k1;  // an extended match length
+        const uint32_t x = x1 & (e * 255);
+        uint32_t slow = ((x >> 7) & k1) * 255;  // extension bytes from 128 up
+        const uint32_t n = lit + 3 * k1 + e + (x & 0x7f7f7f7fu);  // past the offset: 3..146
+        if (m) {  // declined where the match's extension byte is 255
+            LZG_UNROLL
+            for (uint32_t j = 0; j < 4; ++j)
+                if (((m >> (8 * j)) & 1) && in.at(r + j + ((n >> (8 * j)) & 255)) == 255)
+                    slow |= 255u << (8 * j);
+        }
+        return (n + m) | slow;
+    }
+    CDB_HD static uint32_t steps_end(const Staged& in, uint32_t r, uint32_t lim) {
+        uint32_t out = 0;
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t n = hop_rel(in, r + j, lim, 0);
+            out |= (n != kSlowRel && n - r - j < kStepSlow ? n - r - j : kStepSlow) << (8 * j);
+        }
+        return out;
+    }
+    CDB_HD static bool ext_rel(const Staged& in, uint32_t* q, uint32_t* len) {
+        for (uint32_t k = 0; k < kExtCap; ++k) {
+            const uint32_t x = in.at((*q)++);
+            *len += x;
+            if (x != 255) return true;
+        }
+        return false;
+    }
+    // The token's fields: with at most one extension byte per length without
+    // branches, with up to kExtCap in loops. Returns the next token's
+    // position; kSlowRel: the generic forms decide.
+    CDB_HD static uint32_t parse_rel(const Staged& in, uint32_t r, uint32_t lim, Tok* t) {
+        if (r + kMargin > lim) return kSlowRel;
+        const uint32_t u = in.word(r);
+        uint32_t lit = (u >> 4) & 15, ml = (u & 15) + 4;
+        const uint32_t x1 = (u >> 8) & 255, e = lit == 15, m = ml == 19;
+        lit += e ? x1 : 0;
+        uint32_t q = r + 1 + e + lit;
+        if (q + 2 + kExtCap + kSrcSlack <= lim) {
+            const uint32_t v = in.word(q), x2 = (v >> 16) & 255;
+            if (!(e && x1 == 255) && !(m && x2 == 255)) {
+                t->ls = r + 1 + e;
+                t->lit = lit;
+                t->off = v & 0xffff;
+                t->ml = ml + (m ? x2 : 0);
+                return q + 2 + m;
+            }
+        }
+        q = r + 1;
+        lit = (u >> 4) & 15;
+        if (lit == 15 && !ext_rel(in, &q, &lit)) return kSlowRel;
+        t->ls = q;
+        t->lit = lit;
         q += lit;
         if (q + 2 + kExtCap + kSrcSlack > lim) return kSlowRel;
+        t->off = in.at(q) | (in.at(q + 1) << 8);
         q += 2;
-        uint32_t ml = (tok & 15) + 4;
-        if ((tok & 15) == 15 && !ext_rel(b, &q, &ml)) return kSlowRel;
-        *olen = lit + ml;
+        if (ml == 19 && !ext_rel(in, &q, &ml)) return kSlowRel;
+        t->ml = ml;
         return q;
     }
-    // The ladder's answer for such a token when it accepts it as
-    // non-terminal: the ladder's conditions (src/lz4_block.h:139-258) on its
+    // Whether the ladder accepts such a token as non-terminal, `out` bytes
+    // into a batch that has `have` bytes before it and room for `room` (both
+    // clamped below 2^31): its conditions (src/lz4_block.h:139-258) on the
     // final lengths (the extension loops' running checks only fail when the
     // final values fail them); false: the full ladder decides.
-    CDB_HD static bool accept_rel(const uint8_t* b, uint32_t r, uint32_t lim, uint64_t P,
-                                  uint64_t d, uint64_t cap, lzl::Seq* sq) {
-        if (r + kMargin > lim || cap < d) return false;
-        const uint32_t tok = b[r];
-        uint32_t q = r + 1, lit = tok >> 4;
-        if (lit == 15 && !ext_rel(b, &q, &lit)) return false;
-        const uint32_t ls = q;
-        q += lit;  // the offset's position
-        if (q + 2 + kExtCap + kSrcSlack > lim) return false;
-        const uint32_t off = b[q] | (static_cast<uint32_t>(b[q + 1]) << 8);
-        q += 2;
-        uint32_t ml = (tok & 15) + 4;
-        if ((tok & 15) == 15 && !ext_rel(b, &q, &ml)) return false;
-        const uint64_t room = cap - d;
-        if (lit > room || room - lit < kMfLimit || off == 0 || off > d + lit ||
-            ml + kLastLiterals > room - lit)
-            return false;
-        sq->lit_src = P + (ls - r);
-        sq->lit = lit;
-        sq->ml = ml;
-        sq->off = off;
-        sq->next = P + (q - r);
-        sq->done = false;
-        return true;
+    CDB_HD static bool admit(const Tok& t, uint32_t out, uint32_t have, uint32_t room) {
+        const uint32_t used = out + t.lit;
+        return used + kMfLimit <= room && t.off - 1 < have + used &&
+               used + t.ml + kLastLiterals <= room;
     }
 };
 
 // Raw Snappy: one element per step; an element that ends at S steps to S
 // (the chunk's end: Snappy's finish decides there).
 struct SnappyF : lzl::SnappyLadder {
-    static constexpr uint32_t kMaxTok = kTile / 2 + 3;  // elements span >= 2 bytes
+    static constexpr uint32_t kMinStep = 2;  // elements span >= 2 bytes
     static constexpr bool kSnappy = true;
 
     template <class R>
-    CDB_HD static uint64_t step(const R& in, uint64_t S, uint64_t P, uint32_t,
-                                uint64_t* olen) {
+    CDB_HD static uint64_t step(const R& in, uint64_t S, uint64_t P, uint64_t* olen) {
         if (P >= S) return kStepEnd;
         const uint32_t tag = in.at(P);
         const uint32_t kind = tag & 3;
@@ -387,139 +423,96 @@ struct SnappyF : lzl::SnappyLadder {
         if (hdr > S - P) return kStepEnd;
         return P + hdr;
     }
-    template <class R>
-    CDB_HD static uint64_t lit_src(const R& in, uint64_t P, uint64_t) {
-        const uint32_t tag = in.at(P);
-        const uint32_t l6 = tag >> 2;
-        return P + 1 + (l6 >= 60 ? l6 - 59 : 0);
-    }
 
-    // Fast forms over the staged bytes (see Lz4F): elements whose length
-    // is in the tag; copies with 1- or 2-byte offsets.
-    CDB_HD static uint32_t step_rel(const uint8_t* b, uint32_t r, uint32_t lim,
-                                    uint32_t* olen) {
-        const uint32_t tag = b[r];
-        const uint32_t kind = tag & 3, l6 = tag >> 2;
-        uint32_t nx;
-        if (kind == 0) {
-            if (l6 >= 60) return kSlowRel;
-            nx = r + 2 + l6;
-            *olen = l6 + 1;
-        } else if (kind == 3) {
-            return kSlowRel;
-        } else {
-            nx = r + 1 + kind;
-            *olen = kind == 1 ? 4 + (l6 & 7) : l6 + 1;
-        }
-        return nx <= lim ? nx : kSlowRel;
+    // The fast forms (see Lz4F): every element but a literal with a four-byte
+    // length.
+    CDB_HD static uint32_t fields(const Staged& in, uint32_t r, uint32_t* len, uint32_t* u) {
+        *u = in.word(r);
+        const uint32_t kind = *u & 3, l6 = (*u >> 2) & 63;
+        const uint32_t ext = l6 >= 60 ? l6 - 59 : 0;  // bytes of the literal's length
+        const uint32_t n = (ext ? (*u >> 8) & (0xffffffu >> (24 - 8 * (ext & 3))) : l6) + 1;
+        *len = kind == 0 ? n : kind == 1 ? 4 + (l6 & 7) : l6 + 1;
+        if (kind == 0) return ext == 4 ? kSlowRel : r + 1 + ext + n;
+        return r + (kind == 3 ? 5 : 1 + kind);
     }
-    // The ladder's answer (src/snappy_block.h:249-435) for such an element
-    // when it accepts it; false: the full ladder decides.
-    CDB_HD static bool accept_rel(const uint8_t* b, uint32_t r, uint32_t lim, uint64_t P,
-                                  uint64_t d, uint64_t declared, lzl::Seq* sq) {
-        const uint32_t tag = b[r];
-        const uint32_t kind = tag & 3, l6 = tag >> 2;
-        if (kind == 3 || (kind == 0 && l6 >= 60) || declared < d) return false;
-        const uint64_t room = declared - d;
+    CDB_HD static uint32_t steps_rel(const Staged& in, uint32_t r, uint32_t lim) {
+        if (r + 70 > lim) return 0xffffffffu;  // lim <= the chunk's end
+        const uint32_t u = in.word(r);
+        constexpr uint32_t k1 = 0x01010101u;
+        const uint32_t kind = u & 3 * k1, l6 = (u >> 2) & 63 * k1;
+        const uint32_t lit = (((kind | (kind >> 1)) & k1) ^ k1) * 255;  // literals
+        const uint32_t copy = kind + k1 + ((kind >> 1) & kind & k1);    // 2, 3, 5
+        const uint32_t slow = (((l6 + 4 * k1) >> 6) & k1) * 255;        // a length of its own
+        return (lit & ((l6 + 2 * k1) | slow)) | (copy & ~lit);
+    }
+    CDB_HD static uint32_t hop_rel(const Staged& in, uint32_t r, uint32_t lim, uint32_t rest) {
+        if (r + 5 > lim) return kSlowRel;
+        uint32_t len, u;
+        const uint32_t nx = fields(in, r, &len, &u);
+        return nx <= rest ? nx : kSlowRel;  // may lie past the staged bytes
+    }
+    CDB_HD static uint32_t parse_rel(const Staged& in, uint32_t r, uint32_t lim, Tok* t) {
+        if (r + 5 > lim) return kSlowRel;
+        uint32_t len, u;
+        const uint32_t nx = fields(in, r, &len, &u);
+        if (nx > lim) return kSlowRel;
+        const uint32_t kind = u & 3;
         if (kind == 0) {
-            const uint32_t n = l6 + 1;
-            if (r + 1 + n > lim || n > room) return false;
-            sq->lit_src = P + 1;
-            sq->lit = n;
-            sq->ml = 0;
-            sq->off = 0;
-            sq->next = P + 1 + n;
+            t->ls = nx - len;
+            t->lit = len;
+            t->ml = 0;
+            t->off = 1;
         } else {
-            if (r + 1 + kind > lim) return false;
-            uint32_t off, len;
-            if (kind == 1) {
-                off = ((tag >> 5) << 8) | b[r + 1];
-                len = 4 + (l6 & 7);
-            } else {
-                off = b[r + 1] | (static_cast<uint32_t>(b[r + 2]) << 8);
-                len = l6 + 1;
-            }
-            if (off == 0 || off > d || len > room) return false;
-            sq->lit_src = P;
-            sq->lit = 0;
-            sq->ml = len;
-            sq->off = off;
-            sq->next = P + 1 + kind;
+            t->ls = r;
+            t->lit = 0;
+            t->ml = len;
+            t->off = kind == 1   ? ((u & 0xe0) << 3) | ((u >> 8) & 255)
+                     : kind == 2 ? (u >> 8) & 0xffff
+                                 : (u >> 8) | (in.at(r + 4) << 24);
         }
-        sq->done = false;
-        return true;
+        return nx;
+    }
+    // Whether the ladder (src/snappy_block.h:249-435) accepts such an element
+    // (see Lz4F); false: the full ladder decides.
+    CDB_HD static bool admit(const Tok& t, uint32_t out, uint32_t have, uint32_t room) {
+        return out + t.lit + t.ml <= room && (t.ml == 0 || t.off - 1 < have + out);
     }
 };
 
 // ---------------------------------------------------------------------------
-// The tile's token records. LZ4: 32-bit fields, a token's position reused
-// during execution for the in-group part of its match source. Snappy (up to
-// kTile / 2 tokens a tile): 16-bit positions and lengths (lengths saturate:
-// a longer token is a whole-CTA token, re-read by the ladder) and the
-// in-group sources in their own array, so that four CTAs share an SM.
-template <class F, bool Narrow = F::kSnappy>
-struct TokRecs;
-template <class F>
-struct TokRecs<F, false> {
-    static constexpr uint64_t kSat = 0xFFFFFFFFull;
-    uint32_t pos[F::kMaxTok];  // token position - e; executing: its match's in-group source
-    uint32_t lit[F::kMaxTok];  // saturated at kSat
-    uint32_t ml[F::kMaxTok];
-    uint32_t off[F::kMaxTok];
-    uint32_t out[F::kMaxTok];  // output offset - d0
-    CDB_HD uint32_t& dep(uint32_t i, uint32_t) { return pos[i]; }
-};
-template <class F>
-struct TokRecs<F, true> {
-    static constexpr uint64_t kSat = 0xFFFFull;
-    uint16_t pos[F::kMaxTok];  // token position - e (< kTile)
-    uint16_t lit[F::kMaxTok];  // saturated at kSat
-    uint16_t ml[F::kMaxTok];
-    uint32_t off[F::kMaxTok];
-    uint32_t out[F::kMaxTok];       // output offset - d0
-    uint32_t deps[kGroupTok];       // executing: per group token, its match's in-group source
-    CDB_HD uint32_t& dep(uint32_t i, uint32_t g0) { return deps[i - g0]; }
+// What ends a batch early: the first failing or terminal token, the first
+// token that the whole CTA copies.
+struct Cut {
+    uint32_t event, big;
 };
 
-// ---------------------------------------------------------------------------
-// Shared memory of one CTA.
-template <class F>
-struct Shm {
-    static constexpr uint32_t kMaxTok = F::kMaxTok;
-    alignas(16) uint8_t in[kInBytes];  // staged input: positions [ibase, ibase + kInBytes)
+// Shared memory of one CTA. The input is staged in two buffers in turn: the
+// next tile's bytes land while this one's tokens run.
+template <class F, uint32_t kThreads = lzc::kThreads>
+struct Shm : Width<kThreads> {
+    using Width<kThreads>::kTile, Width<kThreads>::kInBytes, Width<kThreads>::kWarps;
+    static constexpr uint32_t kMaxTok = kTile / F::kMinStep + 3;  // tokens of a tile
+    alignas(16) uint8_t in[2][kInBytes];
     union {
-        struct {
-            uint32_t ex[kExIdx];                  // segment exits by position
-            uint8_t rec[kSupers][kSupSegs][kCand];  // [w][segment][lane] entry codes
-            uint32_t cand_exit[kSupers][kCand];
-            uint8_t ovr[kSupers][kSupSegs];       // exact-walk entries
-        } p;
-        TokRecs<F> t;
+        struct {  // finding the tile's tokens
+            uint32_t step[kTile / 4];   // bytes: distance to the next token, kStepSlow
+            uint32_t exit[kTile / 4];   // bytes: distance to the region's exit, kStepSlow
+        } w;
+        struct {  // executing them
+            Rec rec[kThreads];
+            Sector map[kSectors];
+            uint16_t pos[kMaxTok];   // the tile's tokens, relative to its entry
+        } e;
+        uint8_t period[16 * kThreads];  // whole-CTA copies: a short match's period
     } u;
-    alignas(16) uint8_t ring[kRing];
-    uint32_t pend_bits[kGroupOut / 32 + 8];
-    uint32_t seg_entry[kThreads];  // relative entry, or kUnknown for none
-    uint32_t seg_cnt[kThreads];    // tokens; after the scan, the first token's index
-    uint64_t seg_olen[kThreads];   // output bytes; after the scan, the first token's offset
-    uint8_t pend[kThreads];        // per-thread pending match masks
-    uint8_t chosen[kSupers];
-    uint32_t wsum_c[kWarps];  // block scan: per-warp totals
-    uint64_t wsum_o[kWarps];
-    uint32_t first_ev;  // index of the first event token
-    uint8_t ev_kind;
-    int32_t ev_status;
-    uint32_t cut;       // group cut (first big or overflowing token)
-    uint32_t ntok;      // tokens in the tile
-    uint64_t ototal;    // output bytes of the tile's tokens
-    uint64_t tile_exit; // absolute position of the next tile, or kStepEnd
-    uint64_t e;         // tile entry (absolute input position)
-    uint64_t ibase;     // staged input base (absolute position)
-    uint64_t d0;        // output position of the tile's first token
-    uint64_t vlo;       // positions >= vlo are valid in the ring
-    uint64_t flushed;   // positions < flushed are in the destination
-    uint64_t dend;      // output length so far (end of the last executed token)
-    int32_t status;     // chunk status (CUDEC_OK while running)
-    uint32_t finished;  // the chunk is decided
+    uint32_t exit[kThreads];    // region exits
+    uint32_t entry[kThreads];   // region entries (finish), and which regions are entered
+    uint32_t entered[kWarps];
+    uint32_t votes[kWarps];     // settle: threads whose region is not settled
+    int32_t event[kThreads];    // an event token's ladder status (OK: terminal)
+    uint32_t wsum[2][kWarps];   // scans: per-warp totals, used in turn
+    Cut cut[2];                 // batches in turn
+    uint64_t far;               // the successor past 2^31, see kExitFar
 };
 
 // Input reader over the staged tile with the chunk's global bytes behind it
@@ -528,855 +521,528 @@ struct Reader {
     const uint8_t* g;
     const uint8_t* buf;
     uint64_t ibase;
+    uint32_t staged;
     CDB_HD uint32_t at(uint64_t q) const {
         const uint64_t r = q - ibase;
-        return r < kInBytes ? buf[r] : LZC_LDG(g + q);
+        return r < staged ? buf[r] : LZC_LDG(g + q);
     }
 };
-
-CDB_HD uint32_t exi(uint32_t r) { return r + (r >> 4); }  // padded exit index
-
-// ---------------------------------------------------------------------------
-// Ring helpers (positions are output offsets of the chunk).
-struct Ring {
-    uint8_t* ring;
-    uint8_t* dst;
-    uintptr_t dbase;
-    CDB_HD uint32_t idx(uint64_t pos) const {
-        return static_cast<uint32_t>((dbase + pos) & (kRing - 1));
-    }
-    // 16 ring bytes at position a: the five aligned words they touch.
-    CDB_HD V16 get16(uint64_t a) const {
-        constexpr uint32_t kMask = kRing / 4 - 1;
-        const uint32_t ia = idx(a);
-        const uint32_t wi = ia >> 2, sh = (ia & 3) * 8;
-        const uint32_t* r32 = reinterpret_cast<const uint32_t*>(ring);
-        const uint32_t w0 = r32[wi], w1 = r32[(wi + 1) & kMask], w2 = r32[(wi + 2) & kMask];
-        const uint32_t w3 = r32[(wi + 3) & kMask], w4 = r32[(wi + 4) & kMask];
-        return V16{{fsr(w0, w1, sh), fsr(w1, w2, sh), fsr(w2, w3, sh), fsr(w3, w4, sh)}};
-    }
-    // OR the first m (1..16) bytes of v into the ring at position x (the
-    // bytes start at zero and each has one writer).
-    CDB_HD void put16(uint64_t x, const V16& v, uint32_t m) const {
-        const uint32_t ix = idx(x);
-        const uint32_t sh = 8 * (ix & 3);
-        const uint32_t bits = 8 * m;
-        const uint32_t w0 = keep_low(v.w[0], bits);
-        const uint32_t w1 = keep_low(v.w[1], bits > 32 ? bits - 32 : 0);
-        const uint32_t w2 = keep_low(v.w[2], bits > 64 ? bits - 64 : 0);
-        const uint32_t w3 = keep_low(v.w[3], bits > 96 ? bits - 96 : 0);
-        uint32_t* r32 = reinterpret_cast<uint32_t*>(ring);
-        constexpr uint32_t kMask = kRing / 4 - 1;
-        const uint32_t wi = ix >> 2;
-        at_or(r32 + wi, w0 << sh);
-        at_or(r32 + ((wi + 1) & kMask), fsl(w0, w1, sh));
-        at_or(r32 + ((wi + 2) & kMask), fsl(w1, w2, sh));
-        at_or(r32 + ((wi + 3) & kMask), fsl(w2, w3, sh));
-        if (sh) at_or(r32 + ((wi + 4) & kMask), w3 >> (32 - sh));
-    }
-};
-
-// m (1..16) bytes at global address p, read as the aligned words holding
-// them (no word past the last wanted byte is touched).
-CDB_HD V16 gload16(const uint8_t* p, uint32_t m, bool readonly) {
-    const uintptr_t ad = reinterpret_cast<uintptr_t>(p);
-    const uint32_t s4 = static_cast<uint32_t>(ad & 3), sh = 8 * s4;
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(ad - s4);
-    const uint32_t lw = (s4 + m - 1) >> 2;  // last word holding a wanted byte, 0..4
-    uint32_t w[5] = {0, 0, 0, 0, 0};
-    for (uint32_t j = 0; j < 5; ++j)
-        if (j <= lw) w[j] = readonly ? LZC_LDG(q + j) : q[j];
-    return V16{{fsr(w[0], w[1], sh), fsr(w[1], w[2], sh), fsr(w[2], w[3], sh),
-                fsr(w[3], w[4], sh)}};
-}
-
-// m (1..16) staged-or-global input bytes at absolute position a.
-CDB_HD V16 in16(const Reader& in, uint64_t a, uint32_t m) {
-    const uint64_t r = a - in.ibase;
-    if (r < kInBytes && r + m <= kInBytes) {
-        const uint32_t s4 = static_cast<uint32_t>(r & 3), sh = 8 * s4;
-        const uint32_t* q = reinterpret_cast<const uint32_t*>(in.buf + (r - s4));
-        const uint32_t lw = (s4 + m - 1) >> 2;
-        uint32_t w[5] = {0, 0, 0, 0, 0};
-        for (uint32_t j = 0; j < 5; ++j)
-            if (j <= lw && (r - s4) + 4 * j < kInBytes) w[j] = q[j];
-        return V16{{fsr(w[0], w[1], sh), fsr(w[1], w[2], sh), fsr(w[2], w[3], sh),
-                    fsr(w[3], w[4], sh)}};
-    }
-    return gload16(in.g + a, m, true);
-}
-
-// The period expansion of a match with offset off < 16 starting from its
-// first 16 bytes' source (low off bytes of v are the period): the match's
-// first 16 bytes. Every later byte repeats the one rest(off) bytes back.
-CDB_HD V16 period16(const V16& v, uint32_t off) {
-    // Without branches, computed in every lane and selected: periods up to 8
-    // bytes doubled in 64 bits, the next 8 bytes starting r = 8 mod off into
-    // the period; for 9..15 bytes the first 16 - off bytes repeat once.
-    const uint64_t lo = (static_cast<uint64_t>(v.w[1]) << 32) | v.w[0];
-    const uint64_t hi = (static_cast<uint64_t>(v.w[3]) << 32) | v.w[2];
-    const uint32_t d = off < 16 ? off : 16u;
-    const uint32_t sb = 8 * d;  // 8..128
-    uint64_t plo = lo & (~0ull >> ((64 - sb) & 63));
-    plo |= sb < 64 ? plo << (sb & 63) : 0ull;
-    plo |= sb < 32 ? plo << ((2 * sb) & 63) : 0ull;
-    plo |= sb < 16 ? plo << ((4 * sb) & 63) : 0ull;
-    // 8 mod d for d = 1..8, one nibble each
-    const uint32_t r = static_cast<uint32_t>((0x012302000ull >> ((4 * d) & 63)) & 15);
-    const uint64_t phi = (plo >> ((8 * r) & 63)) | (plo << ((8 * (d - r)) & 63));
-    const uint32_t s2 = (sb - 64) & 63;
-    const uint64_t qhi = (hi & ((1ull << s2) - 1)) | (lo << s2);
-    const bool small = d <= 8;
-    const uint64_t olo = small ? plo : lo, ohi = small ? phi : qhi;
-    const V16 e{{static_cast<uint32_t>(olo), static_cast<uint32_t>(olo >> 32),
-                 static_cast<uint32_t>(ohi), static_cast<uint32_t>(ohi >> 32)}};
-    return off < 16 ? e : v;
-}
-CDB_HD uint32_t rest_distance(uint32_t off) {  // off * ceil(16 / off) for off < 16
-    // Q - 16 for off = 1..15, one nibble each
-    return off < 16 ? 16 + static_cast<uint32_t>((0xECA8642052402000ull >> (4 * (off & 15))) & 15)
-                    : off;
-}
 
 // ---------------------------------------------------------------------------
 // The chunk decoder (every thread of the CTA runs it; control flow depends
-// only on shared state read after a barrier).
-template <class F>
+// only on values that every thread holds or that a barrier published).
+template <class F, uint32_t kThreads = lzc::kThreads>
 struct Chunk {
-    Shm<F>& s;
+    using W_ = Width<kThreads>;
+    static constexpr uint32_t kWarps = W_::kWarps, kTile = W_::kTile, kInBytes = W_::kInBytes;
+    static constexpr uint32_t kUnroll = W_::kUnroll, kPart = W_::kPart;
+    static constexpr uint32_t kMaxTok = Shm<F, kThreads>::kMaxTok;
+    template <class V>
+    using Priv = lzc::Priv<V, kThreads>;
+    template <class Fn>
+    CDB_HD static void each(Fn fn) {
+        lzc::each<kThreads>(fn);
+    }
+    template <class Fn>
+    CDB_HD static void each_free(Fn fn) {
+        lzc::each_free<kThreads>(fn);
+    }
+    template <class Fn>
+    CDB_HD static void vote(uint32_t* words, Fn fn) {
+        lzc::vote<kThreads>(words, fn);
+    }
+
+    Shm<F, kThreads>& s;
     const uint8_t* g;  // compressed chunk
     uint64_t S;
     uint8_t* dst;
     uint64_t cap;
-    uint64_t limit;    // LZ4: capacity; Snappy: declared length
-    long long tl = 0;  // profiling builds: thread 0's last phase mark
+    uint64_t limit;      // LZ4: capacity; Snappy: declared length
+    uint64_t e = 0;      // tile entry (absolute input position)
+    uint64_t ibase = 0;  // staged input base (absolute position)
+    uint64_t d = 0;      // output bytes produced
+    uint32_t buf = 0;    // the staging buffer of this tile
+    uint32_t turn = 0, cut_turn = 0;  // which of the alternating buffers are in use
+    long long tl = 0;    // profiling builds: thread 0's last phase mark
 
-    CDB_HD Reader reader() const { return Reader{g, s.in, s.ibase}; }
+    CDB_HD Reader reader() const { return Reader{g, s.in[buf], ibase, kInBytes}; }
     // The staged bytes from the tile entry on, and how many of them the fast
     // forms may read (also bounded by the chunk's end).
-    CDB_HD const uint8_t* staged() const { return s.in + (s.e - s.ibase); }
+    CDB_HD uint32_t staged_at() const { return static_cast<uint32_t>(e - ibase); }
     CDB_HD uint32_t staged_lim() const {
-        const uint64_t avail = kInBytes - (s.e - s.ibase);
-        const uint64_t rest = S > s.e ? S - s.e : 0;
-        return static_cast<uint32_t>(rest < avail ? rest : avail);
+        const uint32_t avail = kInBytes - staged_at();
+        const uint64_t rest = S > e ? S - e : 0;
+        return rest < avail ? static_cast<uint32_t>(rest) : avail;
     }
-    // The exact next position of the chain token at P (or kStepEnd) and its
-    // output length: the fast form when it applies.
-    CDB_HD uint64_t next_of(const Reader& in, const uint8_t* b, uint32_t lim, uint64_t P,
-                            uint64_t* ol) const {
-        if (P >= S) return kStepEnd;
-        const uint64_t r = P - s.e;
-        if (r < lim) {
-            uint32_t o32 = 0;
-            const uint32_t nr = F::step_rel(b, static_cast<uint32_t>(r), lim, &o32);
-            if (nr != kSlowRel) {
-                *ol = o32;
-                return s.e + nr;
-            }
-        }
-        return F::step(in, S, P, 0, ol);
-    }
-    CDB_HD Ring ring() const { return Ring{s.ring, dst, reinterpret_cast<uintptr_t>(dst)}; }
 
-    // ---- 1. stage the tile's input
-    CDB_HD void stage() {
-        each([&](uint32_t tid) {
-            if (tid == 0) {
-                const uint64_t a = (reinterpret_cast<uintptr_t>(g) + s.e) & 15;
-                s.ibase = s.e - a;  // may wrap below zero for the chunk's first block
-            }
-        });
-        const int64_t ib = static_cast<int64_t>(s.ibase);
-        each([&](uint32_t tid) {
-            // aligned blocks holding at least one byte of [0, S) only
-            for (uint32_t b = 16 * tid; b < kInBytes; b += 16 * kThreads) {
+    // Exclusive scan of v over the CTA; returns the total. One barrier.
+    CDB_HD uint32_t scan(Priv<uint32_t>& v, Priv<uint32_t>& excl) {
+        uint32_t total = 0;
+#if CDB_DEVICE_CODE
+        const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        uint32_t* ws = s.wsum[turn];
+        turn ^= 1;
+        uint32_t x = v.v;
+#pragma unroll
+        for (uint32_t k = 1; k < 32; k <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, k);
+            if (lane >= k) x += y;
+        }
+        if (lane == 31) ws[w] = x;
+        __syncthreads();
+        uint32_t before = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kWarps; ++k) {
+            const uint32_t y = ws[k];
+            if (k < w) before += y;
+            total += y;
+        }
+        excl.v = before + x - v.v;
+#else
+        for (uint32_t t = 0; t < kThreads; ++t) {
+            excl[t] = total;
+            total += v[t];
+        }
+#endif
+        return total;
+    }
+
+    // ---- 1. stage the input of the tile at `from` in buffer `to`: aligned
+    // blocks holding at least one byte of [0, S) only; landed by land().
+    CDB_HD static uint64_t base_of(const uint8_t* g, uint64_t from) {
+        return from - ((reinterpret_cast<uintptr_t>(g) + from) & 15);  // may wrap below zero
+    }
+    CDB_HD void stage(uint64_t from, uint32_t to) {
+        const int64_t ib = static_cast<int64_t>(base_of(g, from));
+        each_free([&](uint32_t t) {
+            for (uint32_t b = 16 * t; b < kInBytes; b += 16 * kThreads) {
                 const int64_t q = ib + b;
                 if (q + 16 <= 0 || q >= static_cast<int64_t>(S)) continue;
-                copy16_async(s.in + b, g + q);
+                copy16_async(s.in[to] + b, g + q);
             }
-            land_async();
         });
     }
+    CDB_HD void land() {
+        each([&](uint32_t) { land_async(); });
+    }
 
-    // ---- 2. segment exits
-    CDB_HD void seg_exits() {
-        const Reader in = reader();
-        const uint64_t e = s.e;
-        const uint8_t* b = staged();
-        const uint32_t lim = staged_lim();
+    // The distances to the next token from every position of the tile, by
+    // the format's step (bytes of s.u.w.step; kStepSlow: hop() looks closer).
+    CDB_HD void steps(uint32_t lim) {
+        const Staged in{s.in[buf], staged_at()};
         each([&](uint32_t t) {
-            const uint32_t lo = t * kSeg, hi = lo + kSeg;
-            for (int j = kSeg - 1; j >= 0; --j) {
-                const uint32_t r = lo + static_cast<uint32_t>(j);
-                const uint64_t P = e + r;
-                uint32_t v;
-                uint32_t o32 = 0;
-                const uint32_t fr = r < lim ? F::step_rel(b, r, lim, &o32) : kSlowRel;
-                if (fr != kSlowRel) {
-                    v = fr >= hi ? fr : s.u.p.ex[exi(fr)];
-                } else if (P >= S) {
-                    v = kEndMark;
-                } else {
-                    uint64_t ol = 0;
-                    const uint64_t n = F::step(in, S, P, kExtCap, &ol);
-                    if (n == kStepUnknown) {
-                        v = kUnknown;
-                    } else if (n == kStepEnd) {
-                        v = kEndMark;
-                    } else {
-                        const uint64_t nr = n - e;
-                        if (nr >= hi) v = nr >= kFarRel ? kUnknown : static_cast<uint32_t>(nr);
-                        else v = s.u.p.ex[exi(static_cast<uint32_t>(nr))];
-                    }
-                }
-                s.u.p.ex[exi(r)] = v;
-            }
+            for (uint32_t i = t; i < kTile / 4; i += kThreads)
+                s.u.w.step[i] = F::steps_rel(in, 4 * i, lim);
         });
     }
 
-    // ---- 3. candidate chase, lane k of warp w from position w * kSupPos + k
-    CDB_HD void cand_chase() {
-        each([&](uint32_t tid) {
-            const uint32_t w = tid / 32, k = tid % 32;
-            const uint32_t base = w * kSupPos;
-            uint32_t xr = base + k;
-            for (uint32_t j = 0; j < kSupSegs; ++j) {
-                const uint32_t lo = base + j * kSeg;
-                uint8_t code = kNoEntry;
-                if (xr == kUnknown) {
-                    code = kCodeUnk;
-                } else if (xr == kEndMark) {
-                    code = kCodeEnd;
-                } else if (xr >= lo && xr < lo + kSeg) {
-                    code = static_cast<uint8_t>(xr - lo);
-                    xr = s.u.p.ex[exi(xr)];
-                }
-                s.u.p.rec[w][j][k] = code;
+    // Region t's exits: from each of its positions the distance to the first
+    // chain position past the region (bytes of s.u.w.exit; kStepSlow where a
+    // step on the way is, or the distance is longer). Backwards, kMinStep
+    // positions at a time: none of them leads to another.
+    CDB_HD void exits(uint32_t t) {
+        const uint8_t* step = reinterpret_cast<const uint8_t*>(s.u.w.step);
+        uint8_t* ex = reinterpret_cast<uint8_t*>(s.u.w.exit);
+        const uint32_t lo = t * kReg, hi = lo + kReg;
+        constexpr uint32_t G = F::kMinStep;
+        static_assert(kReg % G == 0 || kReg % G == 1, "whole groups, one position at most left");
+        uint32_t p = hi;
+        while (p >= lo + G) {
+            uint32_t d[G], e[G];
+            LZG_UNROLL
+            for (uint32_t j = 0; j < G; ++j) d[j] = step[p - 1 - j];
+            LZG_UNROLL
+            for (uint32_t j = 0; j < G; ++j) {
+                const uint32_t n = p - 1 - j + d[j];
+                e[j] = n < hi ? ex[n] : 0u;
             }
-            s.u.p.cand_exit[w][k] = xr;
-        });
-    }
-
-    // Exact walk of super-segment w from the relative position xr (inside
-    // it): records the entry of every segment the chain enters; returns the
-    // chain's exit (absolute) or kStepEnd.
-    CDB_HD uint64_t exact_walk(uint32_t w, uint64_t P) {
-        const Reader in = reader();
-        const uint64_t e = s.e;
-        const uint64_t base = e + w * kSupPos, end = base + kSupPos;
-        for (uint32_t j = 0; j < kSupSegs; ++j) s.u.p.ovr[w][j] = kNoEntry;
-        while (P < end) {
-            const uint32_t j = static_cast<uint32_t>((P - base) / kSeg);
-            if (s.u.p.ovr[w][j] == kNoEntry)
-                s.u.p.ovr[w][j] = static_cast<uint8_t>(P - base - j * kSeg);
-            uint64_t ol = 0;
-            const uint64_t n = P >= S ? kStepEnd : F::step(in, S, P, 0, &ol);
-            if (n == kStepEnd) return kStepEnd;
-            P = n;
-        }
-        return P;
-    }
-
-    // ---- 4. tile chase (one thread)
-    CDB_HD void tile_chase() {
-        each([&](uint32_t tid) {
-            if (tid != 0) return;
-            const uint64_t e = s.e;
-            uint64_t P = e;  // the true chain's current position (absolute)
-            for (uint32_t w = 0; w < kSupers; ++w) {
-                const uint64_t base = e + w * kSupPos;
-                if (P == kStepEnd) {
-                    s.chosen[w] = kCodeEnd;
-                    continue;
-                }
-                if (P >= base + kSupPos) {  // no token starts in this super-segment
-                    s.chosen[w] = kNoEntry;
-                    continue;
-                }
-                const uint64_t k = P - base;
-                const uint32_t cx = k < kCand ? s.u.p.cand_exit[w][k] : kUnknown;
-                if (k < kCand && cx != kUnknown) {
-                    s.chosen[w] = static_cast<uint8_t>(k);
-                    P = cx == kEndMark ? kStepEnd : e + cx;
-                } else {
-                    s.chosen[w] = kChoseOvr;
-                    LZC_EVENT(5, 1);
-                    P = exact_walk(w, P);
-                }
+            LZG_UNROLL
+            for (uint32_t j = 0; j < G; ++j) {
+                const uint32_t x = d[j] + e[j];
+                ex[p - 1 - j] = static_cast<uint8_t>(x < kStepSlow ? x : kStepSlow);
             }
-            s.tile_exit = P;
-        });
+            p -= G;
+        }
+        if (p > lo) {
+            const uint32_t d = step[lo], n = lo + d, x = d + (n < hi ? ex[n] : 0u);
+            ex[lo] = static_cast<uint8_t>(x < kStepSlow ? x : kStepSlow);
+        }
     }
 
-    // The entry code of thread t's segment after the tile chase.
-    CDB_HD uint8_t entry_code(uint32_t t) const {
-        const uint32_t w = t / kSupSegs, j = t % kSupSegs;
-        const uint8_t c = s.chosen[w];
-        if (c == kChoseOvr) return s.u.p.ovr[w][j];
-        if (c < kCand) return s.u.p.rec[w][j][c];
-        return kNoEntry;
+    // The step from position p (relative to the tile's entry), which is on
+    // the chain: the next token's relative position or an exit code.
+    CDB_HD uint32_t hop(uint32_t lim, uint32_t rest, uint32_t p) const {
+        const uint32_t d = reinterpret_cast<const uint8_t*>(s.u.w.step)[p];
+        if (d != kStepSlow) return p + d;
+        const Staged in{s.in[buf], staged_at()};
+        const uint32_t n = F::hop_rel(in, p, lim, rest);
+        if (n != kSlowRel) return n;
+        const uint64_t P = e + p;
+        if (P >= S) return kExitEnd;
+        uint64_t ol = 0;
+        const uint64_t nx = F::step(reader(), S, P, &ol);
+        if (nx == kStepEnd) return kExitEnd;
+        if (nx - e < kExitMax) return static_cast<uint32_t>(nx - e);
+        s.far = nx;  // every later region is passed over
+        return kExitFar;
     }
 
-    // Exclusive prefix of the per-segment token counts and output bytes (in
-    // place) and the tile's totals.
-    CDB_HD void scan_counts() {
-#if defined(__CUDA_ARCH__)
-        const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
-        const uint32_t c = s.seg_cnt[t];
-        const uint64_t o = s.seg_olen[t];
-        uint32_t ci = c;
-        uint64_t oi = o;
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            const uint32_t c2 = __shfl_up_sync(0xffffffffu, ci, d);
-            const uint64_t o2 = __shfl_up_sync(0xffffffffu, oi, d);
-            if (lane >= d) {
-                ci += c2;
-                oi += o2;
-            }
-        }
-        if (lane == 31) {
-            s.wsum_c[w] = ci;
-            s.wsum_o[w] = oi;
-        }
-        __syncthreads();
-        uint32_t cb = 0;
-        uint64_t ob = 0;
-        for (uint32_t k = 0; k < w; ++k) {
-            cb += s.wsum_c[k];
-            ob += s.wsum_o[k];
-        }
-        s.seg_cnt[t] = cb + ci - c;
-        s.seg_olen[t] = ob + oi - o;
-        if (t == kThreads - 1) {
-            s.ntok = cb + ci;
-            s.ototal = ob + oi;
-        }
-        __syncthreads();
-#else
-        uint32_t cb = 0;
-        uint64_t ob = 0;
-        for (uint32_t t = 0; t < kThreads; ++t) {
-            const uint32_t c = s.seg_cnt[t];
-            const uint64_t o = s.seg_olen[t];
-            s.seg_cnt[t] = cb;
-            s.seg_olen[t] = ob;
-            cb += c;
-            ob += o;
-        }
-        s.ntok = cb;
-        s.ototal = ob;
-#endif
+    // Where the chain through p leaves region t. Not `sure`: p may not be on
+    // the chain, so a way with an uncommon step is left open.
+    CDB_HD uint32_t leave(uint32_t lim, uint32_t rest, uint32_t t, uint32_t p, bool sure) const {
+        const uint32_t d = reinterpret_cast<const uint8_t*>(s.u.w.exit)[p];
+        if (d != kStepSlow) return p + d;
+        if (!sure) return kExitOpen;
+        while (p < (t + 1) * kReg) p = hop(lim, rest, p);
+        return p;
     }
 
-    // ---- 5. count tokens and output bytes per segment (exact steps)
-    CDB_HD void count() {
-        const Reader in = reader();
-        const uint64_t e = s.e;
-        const uint8_t* b = staged();
-        const uint32_t lim = staged_lim();
+    // The chain from region f on, entered at `sure`: one thread follows it
+    // from region to region.
+    CDB_HD void finish(uint32_t lim, uint32_t rest, uint32_t f, uint32_t sure,
+                       Priv<uint32_t>& entry) {
         each([&](uint32_t t) {
-            const uint8_t c = entry_code(t);
-            uint32_t n = 0;
-            uint64_t ol_sum = 0;
-            uint32_t entry = kUnknown;
-            if (c < kSeg) {
-                entry = t * kSeg + c;
-                uint64_t P = e + entry;
-                const uint64_t hi = e + (t + 1) * kSeg;
-                while (P < hi) {
-                    ++n;
-                    uint64_t ol = 0;
-                    const uint64_t nx = next_of(in, b, lim, P, &ol);
-                    ol_sum += ol;
-                    if (nx == kStepEnd) break;
-                    P = nx;
-                }
-            }
-            s.seg_entry[t] = entry;
-            s.seg_cnt[t] = n;
-            s.seg_olen[t] = ol_sum;
-        });
-        scan_counts();
-    }
-
-    // The ladder's answer for token i of the tile (its position and output
-    // offset from the records): status, and whether it ends the chunk.
-    CDB_HD int ladder_at(uint64_t P, uint64_t d, lzl::Seq* sq) const {
-        *sq = lzl::Seq{};
-        if (F::kSnappy && P == S) {
-            sq->done = true;
-            return F::finish(d, limit);
-        }
-        return F::parse(reader(), S, limit, P, d, sq);
-    }
-
-    // ---- 6. exact ladder per token; records; first event
-    CDB_HD void check() {
-        const Reader in = reader();
-        const uint64_t e = s.e, d0 = s.d0;
-        const uint8_t* b = staged();
-        const uint32_t lim = staged_lim();
-        each([&](uint32_t t) {
-            if (t == 0) s.first_ev = 0xFFFFFFFFu;
-        });
-        each([&](uint32_t t) {
-            const uint32_t entry = s.seg_entry[t];
-            if (entry == kUnknown) return;
-            uint32_t i = s.seg_cnt[t];
-            uint64_t o = s.seg_olen[t];
-            uint64_t P = e + entry;
-            const uint64_t hi = e + (t + 1) * kSeg;
-            while (P < hi) {
-                if (i >= F::kMaxTok || o > 0xFFFFFFFFull) {  // unreachable (tile bounds)
-                    at_min(&s.first_ev, i < F::kMaxTok ? i : F::kMaxTok - 1);
-                    break;
-                }
-                lzl::Seq sq;
-                int st = CUDEC_OK;
-                uint64_t nx, ol;
-                const uint64_t r = P - e;
-                if (r < lim && F::accept_rel(b, static_cast<uint32_t>(r), lim, P, d0 + o, limit,
-                                             &sq)) {
-                    nx = sq.next;
-                    ol = sq.lit + sq.ml;
-                } else {
-                    st = ladder_at(P, d0 + o, &sq);
-                    ol = 0;
-                    nx = next_of(in, b, lim, P, &ol);
-                }
-                constexpr uint64_t kSat = TokRecs<F>::kSat;
-                s.u.t.pos[i] = static_cast<uint32_t>(P - e);
-                s.u.t.lit[i] = static_cast<uint32_t>(sq.lit > kSat ? kSat : sq.lit);
-                s.u.t.ml[i] = static_cast<uint32_t>(sq.ml > kSat ? kSat : sq.ml);
-                s.u.t.off[i] = sq.off;
-                s.u.t.out[i] = static_cast<uint32_t>(o);
-                // the first failing or terminal token ends the chunk; a step
-                // that disagrees with the ladder cannot happen, and would be
-                // reported as an internal error below
-                if (st != CUDEC_OK || sq.done || nx != sq.next) {
-                    at_min(&s.first_ev, i);
-                    break;
-                }
-                ++i;
-                o += ol;
-                P = nx;
-            }
+            if (t < kWarps) s.entered[t] = 0;  // (votes are still being read)
         });
         each([&](uint32_t t) {
             if (t != 0) return;
-            const uint32_t fe = s.first_ev;
-            s.ev_kind = kEvNone;
-            s.ev_status = CUDEC_OK;
-            if (fe == 0xFFFFFFFFu) return;
-            if (fe >= s.ntok) {  // unreachable (tile bounds)
-                s.ev_kind = kEvFail;
-                s.ev_status = CUDEC_ERR_CUDA;
-                return;
+            uint32_t p = sure;
+            while (p < kTile) {
+                const uint32_t r = p / kReg;
+                s.entry[r] = p;
+                s.entered[r / 32] |= 1u << (r % 32);
+                p = leave(lim, rest, r, p, true);
             }
-            lzl::Seq sq;
-            const int st = ladder_at(e + s.u.t.pos[fe], d0 + s.u.t.out[fe], &sq);
-            if (st != CUDEC_OK) {
-                s.ev_kind = kEvFail;
-                s.ev_status = st;
-            } else if (sq.done) {
-                s.ev_kind = kEvDone;
-            } else {
-                s.ev_kind = kEvFail;
-                s.ev_status = CUDEC_ERR_CUDA;
-            }
+            s.exit[kThreads - 1] = p;
+        });
+        each_free([&](uint32_t t) {
+            if (t >= f) entry[t] = (s.entered[t / 32] >> (t % 32)) & 1 ? s.entry[t] : kExitEnd;
         });
     }
 
-    // ---- 7. execution
-    CDB_HD bool is_big(uint32_t i) const {
-        const uint64_t n = static_cast<uint64_t>(s.u.t.lit[i]) + s.u.t.ml[i];
-        return n > kBig;
-    }
-
-    // Copy ring bytes [flushed, end) to the destination: the head up to the
-    // first aligned boundary and, when `fin`, the tail by bytes; whole
-    // aligned 16-byte blocks as vector stores.
-    CDB_HD void flush(uint64_t end, bool fin) {
-        const Ring rg = ring();
-        const uint64_t f = s.flushed;
-        if (end <= f) return;
-        // in addresses: the first aligned boundary at or after f, the last at
-        // or before end (the latter may lie below the former when [f, end)
-        // sits inside one partial block)
-        const uintptr_t db = reinterpret_cast<uintptr_t>(dst);
-        const uintptr_t fa_abs = (db + f + 15) & ~static_cast<uintptr_t>(15);
-        const uintptr_t ea_abs = (db + end) & ~static_cast<uintptr_t>(15);
-        const uint64_t hend = (fa_abs < db + end ? fa_abs : db + end) - db;
-        const bool blocks = ea_abs > fa_abs;
-        const uint64_t fa = fa_abs - db, ea = blocks ? ea_abs - db : hend;
+    // ---- 2.-5. the tile's tokens: their positions in s.u.e.pos, their count,
+    // and the tile's exit (absolute; kStepEnd when the chain ends).
+    CDB_HD uint32_t find_tokens(uint64_t* exit) {
+        const uint32_t lim = staged_lim();
+        const uint64_t left = S - e;
+        const uint32_t rest = left < kExitMax ? static_cast<uint32_t>(left) : kExitMax - 1;
+        steps(lim);
+        LZC_PHASE(1);
+        Priv<uint32_t> entry, next;
         each([&](uint32_t t) {
-            if (f + t < hend) dst[f + t] = rg.ring[rg.idx(f + t)];
-            if (blocks)
-                for (uint64_t b = fa + 16ull * t; b < ea; b += 16ull * kThreads)
-                    st16(dst + b, s.ring + rg.idx(b));
-            if (fin && ea < end && ea + t < end) dst[ea + t] = rg.ring[rg.idx(ea + t)];
+            exits(t);
+            entry[t] = t * kReg;
+            s.exit[t] = leave(lim, rest, t, t * kReg, t == 0);
         });
-        const uint64_t nf = fin ? end : ea;
-        each([&](uint32_t t) {
-            if (t == 0) s.flushed = nf;
-        });
-    }
-
-    // m (1..16) already-written output bytes at position a.
-    CDB_HD V16 fetch16(const Ring& rg, uint64_t a, uint32_t m) const {
-        const uint64_t vlo = s.vlo;
-        if (a >= vlo) return rg.get16(a);
-        if (a + m <= vlo) return gload16(dst + a, m, false);
-        V16 v{{0, 0, 0, 0}};
-        for (uint32_t j = 0; j < m; ++j) {
-            const uint64_t q = a + j;
-            const uint32_t b = q >= vlo ? rg.ring[rg.idx(q)] : dst[q];
-            v.w[j >> 2] |= b << (8 * (j & 3));
-        }
-        return v;
-    }
-
-    CDB_HD void copy_match_ring(const Ring& rg, uint64_t o, uint32_t n, uint32_t off) const {
-        const uint32_t m0 = n < 16 ? n : 16u;
-        rg.put16(o, period16(fetch16(rg, o - off, off < 16 ? off : m0), off), m0);
-        const uint32_t d = rest_distance(off);
-        for (uint32_t k = 16; k < n; k += 16) {
-            const uint32_t m = n - k < 16 ? n - k : 16u;
-            rg.put16(o + k, fetch16(rg, o + k - d, m), m);
-        }
-    }
-
-    // bits [a, b) of the pending map (group-relative output offsets)
-    CDB_HD bool bits_clear(uint32_t a, uint32_t b) const {
-        for (uint32_t w = a >> 5; w <= (b - 1) >> 5; ++w) {
-            uint32_t m = ~0u;
-            if (w == a >> 5) m &= ~0u << (a & 31);
-            if (w == (b - 1) >> 5) m &= ~0u >> (31 - ((b - 1) & 31));
-            if (*static_cast<volatile uint32_t*>(&s.pend_bits[w]) & m) return false;
-        }
-        return true;
-    }
-    CDB_HD void bits_set(uint32_t a, uint32_t b, bool set) {
-        for (uint32_t w = a >> 5; w <= (b - 1) >> 5; ++w) {
-            uint32_t m = ~0u;
-            if (w == a >> 5) m &= ~0u << (a & 31);
-            if (w == (b - 1) >> 5) m &= ~0u >> (31 - ((b - 1) & 31));
-            if (set) at_or(&s.pend_bits[w], m);
-            else at_and(&s.pend_bits[w], ~m);
-        }
-    }
-
-    // Token i's match if its source is ready: copied, then published.
-    CDB_HD bool try_match(const Ring& rg, uint32_t i, uint32_t g0, uint64_t G0) {
-        // the in-group part of its source, packed at the literal phase
-        const uint32_t dep = s.u.t.dep(i, g0);
-        const uint32_t lo = dep & 0xFFFFu, hi = dep >> 16;
-        if (lo < hi && !bits_clear(lo, hi)) return false;
-        const uint32_t lit = s.u.t.lit[i], ml = s.u.t.ml[i], off = s.u.t.off[i];
-        const uint64_t ms = s.d0 + s.u.t.out[i] + lit;
-#if defined(__CUDA_ARCH__)
-        __threadfence_block();  // the source bytes' writers published before their bits cleared
-#endif
-        copy_match_ring(rg, ms, ml, off);
-#if defined(__CUDA_ARCH__)
-        __threadfence_block();  // the bytes land before the bits that publish them
-#endif
-        const uint32_t a = static_cast<uint32_t>(ms - G0);
-        bits_set(a, a + ml, false);
-        return true;
-    }
-
-    // Tokens [g0, g1), all of at most kBig bytes, output [G0, G1) within
-    // kGroupOut: literals, then matches in rounds, through the ring.
-    CDB_HD void exec_group(uint32_t g0, uint32_t g1) {
-        const Reader in = reader();
-        const Ring rg = ring();
-        const uint64_t d0 = s.d0, e = s.e;
-        const uint64_t G0 = d0 + s.u.t.out[g0];
-        const uint64_t G1 = d0 + s.u.t.out[g1 - 1] + s.u.t.lit[g1 - 1] + s.u.t.ml[g1 - 1];
-        // the clear below may zero up to 15 bytes past G1, whose slots held
-        // positions up to G1 + 15 - kRing: those are read back from dst
-        each([&](uint32_t t) {
-            if (t == 0 && G1 + 16 > s.vlo + kRing) s.vlo = G1 + 16 - kRing;
-        });
-        // clear the group's ring bytes and its pending map
-        const uint32_t ib = rg.idx(G0);
-        const uint32_t span = static_cast<uint32_t>(G1 - G0);
-        each([&](uint32_t t) {
-            uint32_t* r32 = reinterpret_cast<uint32_t*>(s.ring);
-            const uint32_t w0 = ib >> 2;
-            if (t == 0) at_and(r32 + w0, (1u << (8 * (ib & 3))) - 1);
-            if (t >= 1 && t < 4 - (w0 & 3)) r32[w0 + t] = 0;
-            const uint32_t end = ib + span;
-            for (uint32_t q = (ib & ~15u) + 16 + 16 * t; q < end; q += 16 * kThreads)
-                zero16(s.ring + (q & (kRing - 1)));
-            for (uint32_t w = t; w < kGroupOut / 32 + 8; w += kThreads) s.pend_bits[w] = 0;
-        });
-        // literals; pending bits of the matches
-        each([&](uint32_t t) {
-            uint8_t pm = 0;
-            for (uint32_t k = 0; k < kPerThread; ++k) {
-                const uint32_t i = g0 + t + k * kThreads;
-                if (i >= g1) break;
-                const uint32_t lit = s.u.t.lit[i], ml = s.u.t.ml[i];
-                const uint64_t o = d0 + s.u.t.out[i];
-                if (lit) {
-                    const uint64_t ls = F::lit_src(in, e + s.u.t.pos[i], lit);
-                    for (uint32_t q = 0; q < lit; q += 16) {
-                        const uint32_t m = lit - q < 16 ? lit - q : 16u;
-                        rg.put16(o + q, in16(in, ls + q, m), m);
-                    }
-                }
-                if (ml) {
-                    const uint32_t a = static_cast<uint32_t>(o + lit - G0);
-                    bits_set(a, a + ml, true);
-                    pm |= static_cast<uint8_t>(1u << k);
-                    // the part of its source inside the group, [lo, hi)
-                    // relative to G0 (empty: every source byte precedes the
-                    // group); the token's position is not needed past here
-                    const uint64_t ms = o + lit, src = ms - s.u.t.off[i];
-                    const uint64_t lo = src > G0 ? src : G0;
-                    const uint64_t hi = src + ml < ms ? src + ml : ms;
-                    s.u.t.dep(i, g0) = lo < hi ? static_cast<uint32_t>(lo - G0) |
-                                                     (static_cast<uint32_t>(hi - G0) << 16)
-                                               : 0u;
-                }
-            }
-            s.pend[t] = pm;
-        });
-        LZC_PHASE(6);
-        LZC_EVENT(3, 1);
-        // matches, as data flow: every thread copies each of its pending
-        // matches once no byte its source reads is still pending, then
-        // publishes it (block fence, then its pending bits cleared). The
-        // lowest pending match of the group is always ready, so every pass
-        // over the CTA makes progress; passes per thread are bounded.
-#if defined(__CUDA_ARCH__)
-        each([&](uint32_t t) {
-            uint8_t pm = s.pend[t];
-            uint32_t spin = 0;
-            for (; pm; ++spin) {
-                // a thread's matches in order (its lowest pending first): a
-                // warp's lanes then hold consecutive tokens and copy together
-                for (uint32_t k = 0; k < kPerThread; ++k)
-                    if (pm & (1u << k)) {
-                        if (try_match(rg, g0 + t + k * kThreads, g0, G0))
-                            pm = static_cast<uint8_t>(pm & ~(1u << k));
-                        break;
-                    }
-                if (pm && spin >= kSpinCap) {  // unreachable: see above
-                    atomicExch(reinterpret_cast<int*>(&s.status), CUDEC_ERR_CUDA);
-                    break;
-                }
-            }
-#ifdef CDB_PHASE_TIMING
-            // one global add per warp (the counts summed across its lanes)
-            const unsigned ws = __reduce_add_sync(0xffffffffu, spin);
-            if ((t & 31) == 0) atomicAdd(&lzc_events[6], static_cast<unsigned long long>(ws));
-#endif
-        });
-#else
-        for (uint32_t pass = 0;; ++pass) {
-            bool any = false;
-            for (uint32_t t = 0; t < kThreads; ++t) {
-                uint8_t pm = s.pend[t];
-                for (uint32_t k = 0; k < kPerThread; ++k)
-                    if ((pm & (1u << k)) && try_match(rg, g0 + t + k * kThreads, g0, G0))
-                        pm = static_cast<uint8_t>(pm & ~(1u << k));
-                s.pend[t] = pm;
-                any = any || pm != 0;
-            }
-            if (!any) break;
-            if (pass > g1 - g0) {  // unreachable: every pass finishes a match
-                s.status = CUDEC_ERR_CUDA;
+        for (uint32_t round = 0;; ++round) {
+            LZC_EVENT(2, 1);
+            vote(s.votes, [&](uint32_t t) {
+                next[t] = t ? s.exit[t - 1] : 0;
+                return next[t] != entry[t] || s.exit[t] == kExitOpen;
+            });
+            uint32_t f = kThreads;  // the first region that is not settled
+            for (uint32_t w = kWarps; w-- > 0;)
+                if (s.votes[w]) f = 32 * w + ctz64(s.votes[w]);
+            if (f == kThreads) break;
+            const uint32_t sure = f ? s.exit[f - 1] : 0;
+            if (round == kRounds) {
+                finish(lim, rest, f, sure, entry);
                 break;
             }
+            each([&](uint32_t t) {
+                const uint32_t hi = (t + 1) * kReg;
+                uint32_t p = next[t];
+                if (t < f) return;
+                if (t > f) {
+                    if (sure >= hi) p = sure;
+                    else if (p >= hi) return;
+                    if (p == entry[t]) return;
+                }
+                entry[t] = p;
+                s.exit[t] = p < hi ? leave(lim, rest, t, p, t == f) : p;
+            });
         }
-#endif
-        LZC_EVENT(2, 1);
-        LZC_PHASE(7);
-        flush(G1, false);
-        each([&](uint32_t t) {
-            if (t == 0) s.dend = G1;
+        LZC_PHASE(2);
+        const uint32_t x = s.exit[kThreads - 1];
+        *exit = x == kExitEnd ? kStepEnd : x == kExitFar ? s.far : e + x;
+        if (*exit < S) stage(*exit, buf ^ 1);  // lands while this tile's tokens run
+        Priv<uint64_t> mask;
+        each_free([&](uint32_t t) {
+            const uint32_t lo = t * kReg;
+            mask[t] = 0;
+            for (uint32_t p = entry[t]; p < lo + kReg; p = hop(lim, rest, p))
+                mask[t] |= 1ull << (p - lo);
         });
-        LZC_PHASE(8);
+        Priv<uint32_t> cnt, at;
+        each_free([&](uint32_t t) { cnt[t] = pop64(mask[t]); });
+        const uint32_t ntok = scan(cnt, at);
+        if (ntok <= kMaxTok)
+            each([&](uint32_t t) {
+                uint32_t i = at[t];
+                for (uint64_t m = mask[t]; m; m &= m - 1)
+                    s.u.e.pos[i++] = static_cast<uint16_t>(t * kReg + ctz64(m));
+            });
+        LZC_PHASE(3);
+        return ntok;
     }
 
-    // One token longer than kBig: the whole CTA copies it straight to the
-    // destination (its exact 64-bit lengths from the ladder).
-    CDB_HD void exec_big(uint32_t i) {
-        const Reader in = reader();
-        const uint64_t P = s.e + s.u.t.pos[i];
-        const uint64_t o = s.d0 + s.u.t.out[i];
+    // The ladder's answer for the token at P with dt bytes before it.
+    CDB_HD int ladder_at(uint64_t P, uint64_t dt, lzl::Seq* sq) const {
+        *sq = lzl::Seq{};
+        if (F::kSnappy && P == S) {
+            sq->done = true;
+            return F::finish(dt, limit);
+        }
+        return F::parse(reader(), S, limit, P, dt, sq);
+    }
+
+    // ---- 6. write the batch's output bytes [y0, y1) that lie in the window
+    // at W (both relative to the batch's first sector, at base), kPart bytes
+    // at a time: kUnroll sectors per warp, then a barrier, so that only the
+    // sources inside a part have to be followed through the map.
+    CDB_HD void copy_window(uint8_t* base, uint32_t y0, uint32_t y1, uint32_t W) {
+        const uint32_t begin = y0 > W ? y0 - W : 0;
+        const uint32_t hi = y1 - W < kWindow ? y1 - W : kWindow;
+        uint8_t* wb = base + W;
+        const uint8_t* in = s.in[buf];
+        for (uint32_t part = begin / kPart * kPart; part < hi; part += kPart) {
+            const uint32_t lo = part > begin ? part : begin;
+            each([&](uint32_t t) {
+                const uint32_t lane = t % 32, k = part / 32 + t / 32;
+                if (32 * k >= hi) return;
+                lzg::Source src[kUnroll];
+                lzg::sources<kUnroll, kThreads>(s.u.e.map, s.u.e.rec, k, kWarps, lane, lo, hi, W,
+                                                src);
+                // literal and match bytes in registers of their own: with one
+                // for both, the second load would wait for the first
+                uint32_t a[kUnroll], m[kUnroll];
+                LZG_UNROLL
+                for (uint32_t j = 0; j < kUnroll; ++j) {
+                    const uint32_t y = 32 * (k + j * kWarps) + lane;
+                    const bool in_range = y - lo < hi - lo;
+                    a[j] = m[j] = 0;
+                    if (in_range && !src[j].lit) m[j] = wb[src[j].at];
+                    if (in_range && src[j].lit) a[j] = in[src[j].at];
+                }
+                LZG_UNROLL
+                for (uint32_t j = 0; j < kUnroll; ++j) {
+                    const uint32_t y = 32 * (k + j * kWarps) + lane;
+                    if (y - lo < hi - lo) wb[y] = static_cast<uint8_t>(src[j].lit ? a[j] : m[j]);
+                }
+            });
+        }
+    }
+
+    // One token longer than kBig (or with literals past the staged input) at
+    // input position P: copied by the whole CTA, its exact 64-bit lengths
+    // from the ladder, which has accepted it. Returns whether it is the
+    // chunk's last.
+    CDB_HD bool exec_big(uint64_t P) {
         lzl::Seq sq;
-        (void)in;
-        (void)ladder_at(P, o, &sq);  // accepted before: the same exact lengths
-        flush(o, true);
-        // literal run: input -> destination
-        const uint64_t lit = sq.lit;
-        const uint64_t ls = sq.lit_src;
-        each([&](uint32_t t) {
-            for (uint64_t q = 16ull * t; q < lit; q += 16ull * kThreads) {
-                const uint32_t m = lit - q < 16 ? static_cast<uint32_t>(lit - q) : 16u;
-                const V16 v = gload16(g + ls + q, m, true);
-                put_global(dst + o + q, v, m);
-            }
-        });
-        // match: waves that never read their own output
-        const uint64_t ms = o + lit, ml = sq.ml;
-        const uint32_t off = sq.off;
-        if (ml) {
-            if (off >= 16 * kThreads) {
-                for (uint64_t wv = 0; wv < ml; wv += 16ull * kThreads) {
+        (void)ladder_at(P, d, &sq);
+        if (sq.lit)
+            each([&](uint32_t t) {
+                lzg::copy_share(dst + d, g + sq.lit_src, sq.lit, t, kThreads);
+            });
+        const uint64_t ms = d + sq.lit, ml = sq.ml, off = sq.off;
+        if (ml && off >= 16 * kThreads) {
+            // waves that never read their own output
+            for (uint64_t k = 0; k < ml; k += off)
+                each([&](uint32_t t) {
+                    lzg::copy_share(dst + ms + k, dst + ms + k - off, ml - k < off ? ml - k : off,
+                                    t, kThreads);
+                });
+        } else if (ml) {
+            const uint32_t f = static_cast<uint32_t>(off);
+            each([&](uint32_t t) {
+                for (uint32_t j = t; j < f; j += kThreads) s.u.period[j] = dst[ms - f + j];
+            });
+            each([&](uint32_t t) {
+                lzg::period_share(dst + ms, s.u.period, f, ml, t, kThreads);
+            });
+        }
+        d = ms + ml;
+        LZC_PHASE(7);
+        LZC_EVENT(4, 1);
+        return sq.done;
+    }
+
+    // Tokens [0, ntok) of the tile. Returns a status, and in *done whether
+    // the chunk's terminal token was among them.
+    CDB_HD int run_tokens(uint32_t ntok, bool* done) {
+        const uint32_t lim = staged_lim();
+        const uint32_t at0 = staged_at();
+        const Staged in{s.in[buf], at0};
+        for (uint32_t b0 = 0; b0 < ntok;) {
+            const uint32_t n = ntok - b0 < kThreads ? ntok - b0 : kThreads;
+            uint8_t* const base = dst + d - ((reinterpret_cast<uintptr_t>(dst) + d) & 31);
+            const uint32_t y0 = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(dst) + d) & 31);
+            constexpr uint32_t kClamp = 0x7fffffffu;
+            const uint32_t have = d < kClamp ? static_cast<uint32_t>(d) : kClamp;
+            const uint32_t room = limit - d < kClamp ? static_cast<uint32_t>(limit - d) : kClamp;
+            Priv<Tok> tok;
+            Priv<bool> fast;
+            Priv<uint32_t> olen, out;
+            // parse; the map starts empty
+            each_free([&](uint32_t t) {
+                for (uint32_t i = t; i < kSectors; i += kThreads) s.u.e.map[i].starts = 0;
+                olen[t] = 0;
+                fast[t] = false;
+                tok[t] = Tok{0, 0, 0, 0};
+                if (t >= n) return;
+                const uint32_t p = s.u.e.pos[b0 + t];
+                if (F::parse_rel(in, p, lim, &tok[t]) != kSlowRel) {
+                    fast[t] = true;
+                    olen[t] = tok[t].lit + tok[t].ml;
+                } else {
+                    // clamped: a token longer than kBig ends the batch
+                    uint64_t ol = 0;
+                    (void)F::step(reader(), S, e + p, &ol);
+                    olen[t] = ol > 65536 ? 65536u : static_cast<uint32_t>(ol);
+                }
+            });
+            const uint32_t total = scan(olen, out);
+            LZC_PHASE(4);
+            Cut& ct = s.cut[cut_turn];
+            Cut& other = s.cut[cut_turn ^ 1];
+            cut_turn ^= 1;
+            each([&](uint32_t t) {
+                if (t == 0) other = Cut{~0u, ~0u};
+                if (t >= n) return;
+                Tok& tk = tok[t];
+                uint32_t ls = tk.ls, off = tk.off, lit = tk.lit, ml = tk.ml;
+                bool big = false;
+                if (!fast[t] || !F::admit(tk, out[t], have, room)) {
+                    lzl::Seq sq;
+                    const uint64_t P = e + s.u.e.pos[b0 + t];
+                    const int st = ladder_at(P, d + out[t], &sq);
+                    uint64_t ol = 0;
+                    const uint64_t nx = P < S ? F::step(reader(), S, P, &ol) : kStepEnd;
+                    bool event = st != CUDEC_OK || sq.done;
+                    s.event[t] = st;
+                    if (!event && nx != sq.next) {  // cannot happen: the steps are the ladder's
+                        s.event[t] = CUDEC_ERR_CUDA;
+                        event = true;
+                    }
+                    if (event) at_min(&ct.event, t);
+                    big = sq.lit && (sq.lit_src - e > lim || sq.lit > lim - (sq.lit_src - e));
+                    big = big || sq.lit > kBig || sq.ml > kBig;
+                    lit = big ? 0 : static_cast<uint32_t>(sq.lit);
+                    ml = big ? 0 : static_cast<uint32_t>(sq.ml);
+                    off = sq.off;
+                    ls = static_cast<uint32_t>(sq.lit_src - e);
+                }
+                big = big || lit + ml > kBig || off >> 31;  // the gather's limits
+                const uint32_t y = y0 + out[t];
+                const uint32_t le = y + lit;
+                s.u.e.rec[t] = Rec{y, le, at0 + ls - y, off};
+                if (big) at_min(&ct.big, t);
+                else lzg::map_token(s.u.e.map, t, y, le + ml, 0);
+                if (t == 0) s.u.e.map[0].before = 0;
+            });
+            const uint32_t ev = ct.event, bg = ct.big;
+            LZC_PHASE(5);
+            LZC_EVENT(3, 1);
+            // tokens [0, k) are gathered; then the event or the big token
+            uint32_t k = ev < bg ? ev : bg;
+            if (k > n) k = n;
+            const bool at_event = ev == k && k < n;
+            if (at_event && s.event[k] != CUDEC_OK) return s.event[k];
+            const bool last = at_event && bg != k;  // terminal, gathered with the batch
+            const uint32_t y1 = last     ? s.u.e.rec[k].le
+                                : k == 0 ? y0
+                                : k < n  ? s.u.e.rec[k].out
+                                         : y0 + total;
+            for (uint32_t W = 0; y1 > y0 && W < y1; W += kWindow) {
+                if (W) {
                     each([&](uint32_t t) {
-                        const uint64_t q = wv + 16ull * t;
-                        if (q >= ml) return;
-                        const uint32_t m = ml - q < 16 ? static_cast<uint32_t>(ml - q) : 16u;
-                        put_global(dst + ms + q, gload16(dst + ms + q - off, m, false), m);
+                        for (uint32_t i = t; i < kSectors; i += kThreads) s.u.e.map[i].starts = 0;
+                    });
+                    each([&](uint32_t t) {
+                        if (t < k || (last && t == k)) {
+                            const uint32_t end = t + 1 < n ? s.u.e.rec[t + 1].out : y0 + total;
+                            lzg::map_token(s.u.e.map, t, s.u.e.rec[t].out, t == k ? y1 : end, W);
+                        }
                     });
                 }
-            } else {
-                // the period (off < 4096 bytes) in the ring, then each byte is
-                // period[(x - ms) mod off]
-                each([&](uint32_t t) {
-                    for (uint32_t j = t; j < off; j += kThreads) s.ring[j] = dst[ms - off + j];
-                });
-                each([&](uint32_t t) {
-                    for (uint64_t q = 16ull * t; q < ml; q += 16ull * kThreads) {
-                        const uint32_t m = ml - q < 16 ? static_cast<uint32_t>(ml - q) : 16u;
-                        uint32_t ph = static_cast<uint32_t>(q % off);
-                        V16 v{{0, 0, 0, 0}};
-                        for (uint32_t j = 0; j < m; ++j) {
-                            v.w[j >> 2] |= static_cast<uint32_t>(s.ring[ph]) << (8 * (j & 3));
-                            ph = ph + 1 == off ? 0 : ph + 1;
-                        }
-                        put_global(dst + ms + q, v, m);
-                    }
-                });
+                copy_window(base, y0, y1, W);
+                LZC_EVENT(5, 1);
             }
-        }
-        const uint64_t end = ms + ml;
-        each([&](uint32_t t) {
-            if (t == 0) {
-                s.flushed = end;
-                s.vlo = end;
-                s.dend = end;
+            LZC_PHASE(6);
+            d += y1 - y0;
+            if (last) {
+                *done = true;
+                return CUDEC_OK;
             }
-        });
-        LZC_PHASE(9);
-        LZC_EVENT(4, 1);
-    }
-
-    CDB_HD void execute(uint32_t ne) {
-        uint32_t g0 = 0;
-        while (g0 < ne && s.status == CUDEC_OK) {
-            // the group: up to kGroupTok tokens, cut at a big token or where
-            // the output passes kGroupOut
-            const uint32_t lim = ne - g0 < kGroupTok ? ne : g0 + kGroupTok;
-            const uint32_t o0 = s.u.t.out[g0];
-            each([&](uint32_t t) {
-                if (t == 0) s.cut = lim;
-            });
-            each([&](uint32_t t) {
-                for (uint32_t i = g0 + t; i < lim; i += kThreads) {
-                    const uint64_t end = static_cast<uint64_t>(s.u.t.out[i]) - o0 +
-                                         s.u.t.lit[i] + s.u.t.ml[i];
-                    if (is_big(i) || end > kGroupOut) {
-                        at_min(&s.cut, i);
-                        break;
-                    }
+            if (k < n) {
+                const uint64_t P = e + s.u.e.pos[b0 + k];
+                if (exec_big(P)) {
+                    *done = true;
+                    return CUDEC_OK;
                 }
-            });
-            const uint32_t c = s.cut;
-            LZC_PHASE(10);
-            if (c == g0) {
-                exec_big(g0);
-                g0 += 1;
+                b0 += k + 1;
             } else {
-                exec_group(g0, c);
-                g0 = c;
+                b0 += n;
             }
         }
+        return CUDEC_OK;
     }
 
     // ---- the chunk
     CDB_HD int run(uint64_t* written) {
+        const int st = decode(written);
+        // a chunk may end with the next tile's copies in flight
+        each_free([&](uint32_t) { land_async(); });
+        return st;
+    }
+    CDB_HD int decode(uint64_t* written) {
         uint64_t first = 0, lim = 0;
-        int st = F::begin(Reader{g, s.in, ~0ull >> 1}, S, cap, &first, &lim);
+        const int st = F::begin(Reader{g, s.in[0], ~0ull >> 1, 0}, S, cap, &first, &lim);
         if (st != CUDEC_OK) return st;
         limit = lim;
-        each([&](uint32_t t) {
-            if (t == 0) {
-                s.e = first;
-                s.d0 = 0;
-                s.vlo = 0;
-                s.flushed = 0;
-                s.dend = 0;
-                s.status = CUDEC_OK;
-                s.finished = 0;
-            }
+        e = first;
+        each_free([&](uint32_t t) {  // published by the first tile's barriers
+            if (t == 0) s.cut[0] = s.cut[1] = Cut{~0u, ~0u};
         });
         // every tile holds at least one token and consumes at least one
         // position, so the chunk's tiles number at most S + 1
         uint64_t fuel = S == ~0ull ? ~0ull : S + 1;
         LZC_START();
+        stage(e, 0);
         for (;;) {
-            stage();
+            ibase = base_of(g, e);
+            land();
             LZC_PHASE(0);
-            seg_exits();
-            LZC_PHASE(1);
-            cand_chase();
-            LZC_PHASE(2);
-            tile_chase();
-            LZC_PHASE(3);
-            count();
-            LZC_PHASE(4);
-            if (s.ntok > F::kMaxTok) return CUDEC_ERR_CUDA;  // unreachable (tile bounds)
-            check();
-            LZC_PHASE(5);
+            uint64_t exit = 0;
+            const uint32_t ntok = find_tokens(&exit);
+            if (ntok > kMaxTok) return CUDEC_ERR_CUDA;  // unreachable (tile bounds)
             LZC_EVENT(0, 1);
-            LZC_EVENT(1, s.ntok);
-            const uint32_t fe = s.first_ev;
-#ifdef LZC_TRACE
-            LZC_TRACE(s.e, s.d0, s.ntok, s.ototal, fe, s.ev_kind, s.ev_status, s.tile_exit);
-            if (fe != 0xFFFFFFFFu && s.ev_kind == kEvFail) LZC_TRACE_SEGS(s);
-#endif
-            if (fe != 0xFFFFFFFFu && s.ev_kind == kEvFail) return s.ev_status;
-            const uint32_t ne = fe != 0xFFFFFFFFu ? fe + 1 : s.ntok;
-            execute(ne);
-            if (s.status != CUDEC_OK) return s.status;
-            if (fe != 0xFFFFFFFFu) break;  // terminal token executed
-            if (s.tile_exit == kStepEnd || fuel-- == 0) return CUDEC_ERR_CORRUPT_INPUT;
-            const uint64_t nd = s.d0 + s.ototal;
-            const uint64_t ne_pos = s.tile_exit;
-            each([&](uint32_t t) {
-                if (t == 0) {
-                    s.e = ne_pos;
-                    s.d0 = nd;
-                }
-            });
+            LZC_EVENT(1, ntok);
+            bool done = false;
+            const int rt = run_tokens(ntok, &done);
+            if (rt != CUDEC_OK) return rt;
+            if (done) break;
+            if (exit == kStepEnd || fuel-- == 0) return CUDEC_ERR_CORRUPT_INPUT;
+            e = exit;
+            buf ^= 1;
         }
-        const uint64_t d = s.dend;
-        flush(d, true);
         *written = d;
         return CUDEC_OK;
     }
 };
 
-
 // ---------------------------------------------------------------------------
-// The batch kernel: one CTA per chunk at a time, persistent grid-stride over
-// the batch. Dynamic shared memory: sizeof(Shm<F>).
+// The batch kernel: one CTA per chunk. Dynamic shared memory: sizeof(Shm).
 #if defined(__CUDACC__)
-template <class F>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+template <class F, uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads, Width<kThreads>::kPerSm)
     lz_cta_kernel(const void* const* src_ptrs, const size_t* src_sizes, void* const* dst_ptrs,
                   const size_t* dst_caps, size_t n, cudec_chunk_result* results) {
     extern __shared__ __align__(16) uint8_t lzc_smem[];
-    Shm<F>& s = *reinterpret_cast<Shm<F>*>(lzc_smem);
+    Shm<F, kThreads>& s = *reinterpret_cast<Shm<F, kThreads>*>(lzc_smem);
     for (size_t c = blockIdx.x; c < n; c += gridDim.x) {
-        Chunk<F> ch{s, static_cast<const uint8_t*>(src_ptrs[c]), src_sizes[c],
-                    static_cast<uint8_t*>(dst_ptrs[c]), dst_caps[c], 0};
+        Chunk<F, kThreads> ch{s, static_cast<const uint8_t*>(src_ptrs[c]), src_sizes[c],
+                              static_cast<uint8_t*>(dst_ptrs[c]), dst_caps[c], 0};
         uint64_t written = 0;
         const int st = ch.run(&written);
         if (threadIdx.x == 0) {

@@ -56,12 +56,11 @@ constexpr uint32_t kSmem = kWarps * kWarpSmem;
 constexpr int kBuckets = CUDEC_MIXED_BUCKETS;
 constexpr int kSizeClasses = 64;  // floor(log2(capacity)) classes for the order
 constexpr int kClasses = 2 * kSizeClasses;  // CTA-decoded chunks: the upper half
-constexpr uint32_t kCtaWarps = lzc::kWarps;  // warps per chunk of the CTA decoder
-// Resident CTAs per SM of the CTA grid, at most: three leave room for the
-// warp grid that decodes beside it (with four, which the shared memory
-// allows, 30,000 uneven LZ4 + Snappy chunks took 7 % longer).
-constexpr int kCtaPerSmMax = 3;
-static_assert(kCtaWarps == CUDEC_MIXED_CTA_WARPS, "the ABI's whole-CTA warps value");
+// The shape value that names the CTA decoder (its own width is lzc::kThreads).
+constexpr uint32_t kCtaWarps = CUDEC_MIXED_CTA_WARPS;
+// Resident CTAs per SM of the CTA grid, at most: they leave room for the warp
+// grid that decodes beside it.
+constexpr int kCtaPerSmMax = 5;
 constexpr uint32_t kCtaSmem = kMaxOf(static_cast<uint32_t>(sizeof(lzc::Shm<lzc::Lz4F>)),
                                      static_cast<uint32_t>(sizeof(lzc::Shm<lzc::SnappyF>)));
 static_assert(kWarpSmem % 16 == 0, "per-warp regions stay 16-byte aligned");
@@ -159,7 +158,8 @@ struct CtaArgs {
     Ctrl* ctrl;
 };
 
-__global__ void __launch_bounds__(lzc::kThreads, lzc::kCtasPerSm) mixed_cta_kernel(CtaArgs a) {
+__global__ void __launch_bounds__(lzc::kThreads, lzc::Width<lzc::kThreads>::kPerSm)
+    mixed_cta_kernel(CtaArgs a) {
     extern __shared__ __align__(16) uint8_t cta_smem[];
     __shared__ unsigned long long claim;
     const unsigned long long ncta = a.ctrl->ncta;

@@ -1,0 +1,48 @@
+// Host emulation of the CTA-per-chunk LZ decoder's device path
+// (cudec_b200/csrc/lz_cta_kernel.cuh): the source itself with its warps and
+// barriers run by cuda_emul.h, at each of the kernel's widths. Test
+// infrastructure only.
+#include "cuda_emul.h"
+
+#include "lz_cta_kernel.cuh"
+
+namespace {
+
+template <class F, uint32_t T>
+int run(const uint8_t* src, uint64_t S, uint8_t* dst, uint64_t cap, uint64_t seed,
+        uint64_t* written) {
+    using Shm = cdb::lzc::Shm<F, T>;
+    static Shm* shm = new Shm();
+    std::memset(static_cast<void*>(shm), 0x5C, sizeof *shm);  // stale state must not matter
+    std::vector<int> st(T, -2);
+    std::vector<uint64_t> out(T, 0);
+    const bool ok = emul::run(T, seed, [&] {
+        const uint32_t t = threadIdx.x;
+        cdb::lzc::Chunk<F, T> ch{*shm, src, S, dst, cap, 0};
+        uint64_t w = 0;
+        st[t] = ch.run(&w);
+        out[t] = w;
+    });
+    for (uint32_t t = 1; ok && t < T; ++t)
+        if (st[t] != st[0] || (st[0] == 0 && out[t] != out[0])) return -3;  // threads disagree
+    *written = ok && st[0] == 0 ? out[0] : 0;
+    return ok ? st[0] : -1;
+}
+
+template <class F>
+int widths(uint32_t threads, const uint8_t* src, uint64_t S, uint8_t* dst, uint64_t cap,
+           uint64_t seed, uint64_t* written) {
+    return threads == 128   ? run<F, 128>(src, S, dst, cap, seed, written)
+           : threads == 256 ? run<F, 256>(src, S, dst, cap, seed, written)
+                            : run<F, 512>(src, S, dst, cap, seed, written);
+}
+
+}  // namespace
+
+// fmt 0 = LZ4, 1 = Snappy; -1: the CTA deadlocks or its lanes meet different
+// collectives.
+extern "C" int lz_emulate(int fmt, uint32_t threads, const uint8_t* src, uint64_t n, uint8_t* dst,
+                          uint64_t cap, uint64_t seed, uint64_t* written) {
+    return fmt == 0 ? widths<cdb::lzc::Lz4F>(threads, src, n, dst, cap, seed, written)
+                    : widths<cdb::lzc::SnappyF>(threads, src, n, dst, cap, seed, written);
+}

@@ -1,0 +1,116 @@
+"""The decoders' device source, run on the CPU.
+
+tests/native/cuda_emul.h runs a CTA's threads as fibers that meet at warp
+collectives and barriers (a deadlock, lanes at different collectives, or
+threads that disagree on the result fail the run), in an order drawn from a
+seed. The sizes are those where the decoders change their way: LZ4 and Snappy
+chunks of one tile and of several at each width of the CTA, batches cut by
+long tokens, tiles that few tokens settle. Statuses, bytes and untouched
+memory around them equal the oracle's; the mutants cover the early ends.
+"""
+import ctypes
+import os
+import random
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle
+from cudec_b200 import workload as W
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+CSRC = os.path.join(ROOT, "cudec_b200", "csrc")
+
+
+def _build(name):
+    out_dir = os.path.join(HERE, "native", "_build")
+    os.makedirs(out_dir, exist_ok=True)
+    so = os.path.join(out_dir, "lib%s.so" % name)
+    src = os.path.join(HERE, "native", name + ".cpp")
+    deps = [src, os.path.join(HERE, "native", "cuda_emul.h")] + [
+        os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
+    if not os.path.exists(so) or any(os.path.getmtime(d) > os.path.getmtime(so) for d in deps):
+        subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-w",
+                        "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, src, "-o", so],
+                       check=True)
+    return ctypes.CDLL(so)
+
+
+@pytest.fixture(scope="module")
+def lz():
+    lib = _build("lz_emul")
+    lib.lz_emulate.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_uint64,
+                               ctypes.c_void_p, ctypes.c_uint64, ctypes.c_uint64,
+                               ctypes.POINTER(ctypes.c_uint64)]
+
+    def call(fmt, threads):
+        return lambda src, n, dst, cap, seed, written: lib.lz_emulate(
+            fmt, threads, src, n, dst, cap, seed, written)
+    return call
+
+
+def check(run, want, comp, cap, seed=0, skew=0, label=None):
+    src = np.zeros(len(comp) + 64 + skew, dtype=np.uint8)
+    src[32 + skew:32 + skew + len(comp)] = np.frombuffer(comp, dtype=np.uint8)
+    dst = np.full(cap + 96, 0xA5, dtype=np.uint8)
+    o = 32 + (skew * 7) % 32
+    w = ctypes.c_uint64(0)
+    st = run(src.ctypes.data + 32 + skew, len(comp), dst.ctypes.data + o, cap, seed,
+             ctypes.byref(w))
+    want_st, want_out = want(comp, cap)
+    assert st == want_st, (label, st, want_st, len(comp), cap, seed)
+    assert (dst[:o] == 0xA5).all() and (dst[o + cap:] == 0xA5).all(), (label, "out of bounds")
+    if st == 0:
+        assert dst[o:o + w.value].tobytes() == want_out, (label, "bytes differ")
+        assert (dst[o + w.value:o + cap] == 0xA5).all(), (label, "wrote past bytes_written")
+
+
+def mutate(rng, comp):
+    b = bytearray(comp)
+    for _ in range(rng.randrange(1, 4)):
+        r = rng.random()
+        if r < 0.75:
+            b[rng.randrange(len(b))] ^= 1 << rng.randrange(8)
+        elif r < 0.9:
+            b = b[:rng.randrange(1, len(b) + 1)]
+        else:
+            b += rng.randbytes(rng.randrange(1, 5))
+    return bytes(b)
+
+
+def contents(size):
+    rng = random.Random(size)
+    yield W.generate([max(size, 1)], W.lz_params(), seeds=[size])[0][:size].tobytes()
+    yield bytes(size)
+    yield rng.randbytes(size)
+    yield (b"the quick brown fox jumps over the lazy dog; " * (size // 45 + 1))[:size]
+    # long runs of either kind between short ones
+    parts = [rng.randbytes(rng.randrange(1, 2500)) + b"x" * rng.randrange(1, 2500)
+             for _ in range(size // 2500 + 1)]
+    yield (b"".join(parts) + parts[0] * 3)[:size]
+
+
+def lz_contents(size):
+    rng = random.Random(size)
+    for p in (0.1, 0.5, 0.9):
+        yield W.generate([max(size, 1)], W.lz_params(p), seeds=[size])[0][:size].tobytes()
+    words = [rng.randbytes(rng.randrange(3, 12)) for _ in range(200)]
+    yield b"".join(rng.choice(words) for _ in range(size // 5 + 1))[:size]
+
+
+# One tile holds 52 positions per thread.
+@pytest.mark.parametrize("threads", [128, 256, 512])
+@pytest.mark.parametrize("size", [0, 1, 13, 129, 1025, 6656, 30000])
+def test_lz(lz, size, threads):
+    rng = random.Random(size)
+    datas = list(lz_contents(size)) + list(contents(size))[1:]
+    for k, data in enumerate(datas):
+        for fmt, pack, want in ((0, W.lz4_compress, oracle.lz4_decode),
+                                (1, W.snappy_compress, oracle.snappy_decode)):
+            f = pack(data)
+            check(lz(fmt, threads), want, f, size, k + 1, (5 * k + fmt) % 16, (size, k, fmt))
+            for m in range(4 if size < 6000 else 1):
+                check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2, m, 0,
+                      (size, k, fmt, m))

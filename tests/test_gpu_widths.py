@@ -1,0 +1,63 @@
+"""GPU parity of the LZ4 / Snappy batch entries at each width of their CTAs
+(512, 256 and 128 threads per chunk, by the batch's chunks per SM), on chunks
+whose sizes and tokens sit at the decoder's edges: a region, a tile and the
+tiles past it, runs at and past what a lane, a warp and the whole CTA copy.
+Every status, byte and untouched tail equals the oracle's.
+"""
+import random
+
+import pytest
+
+import oracle
+from cudec_b200 import workload as W
+from cudec_b200.device import DeviceBatch
+
+pytestmark = pytest.mark.gpu
+
+PACK = {"lz4": W.lz4_compress, "snappy": W.snappy_compress}
+WANT = {"lz4": oracle.lz4_decode, "snappy": oracle.snappy_decode}
+
+
+def chunks(n):
+    rng = random.Random(n)
+    runs = (1, 15, 16, 17, 31, 32, 127, 128, 129, 1023, 1024, 1025, 5000)
+    out = []
+    for i in range(n):
+        size = (1, 52, 53, 6656, 6657, 13312, 26624, 40000)[i % 8]
+        kind = i // 8 % 4
+        if kind == 0:
+            data = W.generate([size], W.lz_params(0.5), seeds=[i])[0].tobytes()
+        elif kind == 1:  # runs of random and repeated bytes, each copied again later
+            parts = [rng.randbytes(runs[k % 13]) + bytes([k % 7]) * runs[(k + i) % 13]
+                     for k in range(60)]
+            data = (b"".join(parts) * 2)[:size]
+        elif kind == 2:  # few tokens per tile
+            data = W.generate([size], W.lz_params(0.02), seeds=[i])[0].tobytes()
+        else:
+            data = (rng.randbytes(1 + i % 40) * size)[:size]
+        out.append(data)
+    return out
+
+
+@pytest.mark.parametrize("fmt", ["lz4", "snappy"])
+@pytest.mark.parametrize("n", [32, 200, 500])
+def test_widths(cuda, fmt, n):
+    import torch
+    raws = chunks(n)
+    comps = [PACK[fmt](r) for r in raws]
+    rng = random.Random(5)
+    for i in range(0, n, 11):  # some mutants among them
+        b = bytearray(comps[i])
+        b[rng.randrange(len(b))] ^= 1 << rng.randrange(8)
+        comps[i] = bytes(b)
+    caps = [len(r) for r in raws]
+    b = DeviceBatch(comps, caps, device=cuda, dst_align=16, dst_skew=3, src_skew=5)
+    assert b.run(fmt) == 0
+    torch.cuda.synchronize()
+    res, dst = b.results(), b.dst_host()
+    for i in range(n):
+        st, out = WANT[fmt](comps[i], caps[i])
+        assert res[i]["status"] == st, (i, res[i], st)
+        if st == 0:
+            assert res[i]["bytes_written"] == len(out)
+            assert b.output(i, dst) == out + b"\xa5" * (caps[i] - len(out)), i
