@@ -19,7 +19,9 @@ namespace gdf {
 constexpr uint32_t kWarps = 4;
 constexpr int kSmem = static_cast<int>(kWarps * sizeof(Tables));
 
-__global__ void __launch_bounds__(32 * kWarps)
+constexpr int kCtasPerSm = 7;  // resident CTAs per SM the registers allow
+
+__global__ void __launch_bounds__(32 * kWarps, kCtasPerSm)
     gdeflate_kernel(const void* const* src_ptrs, const size_t* src_sizes, void* const* dst_ptrs,
                     const size_t* dst_caps, size_t n, cudec_chunk_result* results) {
     extern __shared__ __align__(16) uint8_t gdf_smem[];

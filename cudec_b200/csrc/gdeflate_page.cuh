@@ -15,11 +15,21 @@
 // memory, canonical decoding for longer codes; the precode has a complete
 // 7-bit table. End-of-block quiesce is a ballot: lanes after the first lane
 // that read end-of-block (and have no distance pending) do not consume.
-// Output positions come from a warp scan of the round's item lengths; bytes
-// go straight to the destination (a page is at most 64 KiB) and copies read
-// them back from there. Shared memory holds only the tables (about 6 KB per
-// warp), so many pages decode per SM: staging the page in shared memory
-// measured 5x slower for lack of resident warps.
+// Output positions come from a warp scan of the round's item lengths. A
+// literal goes straight to the destination; a match is queued once its
+// distance is known, and the queue is executed a match per lane when it holds
+// 32 (lane_copy.cuh): a round yields some three matches, which on their own
+// left most lanes idle while the warp waited for memory once per 16 bytes of
+// the longest. Shared memory holds only the tables and the queue, so many
+// pages decode per SM: staging the page in shared memory measured 5x slower
+// for lack of resident warps.
+//
+// Bound by instruction issue and, in small batches, by one page's chain of
+// rounds; memory is far from it. 4,096 pages of 64 KiB took 2,241 us with
+// copies made in each round, the input refilled by per-lane loads, serial
+// table builds and long codes walked bit by bit; 1,820 with the queue, the
+// refill from a register window, lane-parallel builds and long codes found by
+// five compares. 24 pages: 999 and 885 us.
 //
 // Errors are reported in serial order: an operation's error at lane l
 // precedes lane l's refill, which precedes lane l+1's operation.
@@ -28,7 +38,7 @@
 #include <cstdint>
 
 #include "cudec.h"
-#include "lz_warp_kernel.cuh"
+#include "lane_copy.cuh"
 
 namespace cdb {
 namespace gdf {
@@ -37,21 +47,36 @@ constexpr uint32_t kPageMax = 65536;
 constexpr uint32_t kTabBits = 10;
 constexpr uint32_t kNoEvent = 64;  // event index when none (2 * lane + phase otherwise)
 
-// Per-warp decode tables (shared memory).
-struct __align__(16) Tables {
-    uint16_t ltab[1 << kTabBits];  // sym | len << 9, 0 = use the canonical path
-    uint16_t dtab[1 << kTabBits];
-    uint16_t ptab[128];
-    uint16_t lcount[16], dcount[16];
-    uint16_t lsym[288], dsym[32];
-    uint16_t code[320];  // canonical codes during a table build
-    uint8_t lens[320];
-    uint8_t plen[20];
-    // canonical-decode state after the lengths the lookup table covers
-    // (first code and symbol index at length kTabBits + 1), per table
-    int32_t lfirst, lindex, dfirst, dindex;
-};
+constexpr uint32_t kQueue = 64;      // queued matches: up to a round's 32 past half of it
 
+// Per-warp shared memory: decode tables, then what building them needs, or
+// the match queue and its map.
+struct __align__(16) Tables {
+    // symbol | length << 9, 0: longer than the table (or no code)
+    uint16_t ltab[1 << kTabBits];
+    uint16_t dtab[1 << kTabBits];
+    uint16_t count[16];  // symbols per length during a table build
+    uint16_t lsym[288], dsym[32];
+    uint32_t base[64];  // lengths' (from 0) and distances' (from 32) base | extra bits << 24
+    union {
+        struct {
+            uint16_t ptab[128];
+            uint16_t next[16], place[16];
+            uint8_t lens[320];
+            uint8_t plen[20];
+        } b;
+        struct {
+            uint32_t at[kQueue], len[kQueue], off[kQueue];
+            uint8_t period[lanes::kPeriod];  // a long match's period
+        } q;
+    } u;
+    // codes longer than the table: see Long
+    struct Long {
+        uint16_t limit[5];  // of length kTabBits + 1 + k, left-aligned in 15 bits: past its codes
+        uint16_t from[5];   // its first code, left-aligned the same
+        uint16_t index[5];  // its first symbol's place in sym
+    } llong, dlong;
+};
 
 static __constant__ uint16_t kLBase[29] = {3,  4,  5,  6,  7,  8,  9,  10,  11,  13,
                                     15, 17, 19, 23, 27, 31, 35, 43,  51,  59,
@@ -67,18 +92,40 @@ static __constant__ uint8_t kDExtra[32] = {0, 0, 0, 0, 1, 1, 2, 2, 3,  3,  4,  4
 static __constant__ uint8_t kPerm[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 11, 12, 13, 14, 15, 5, 4, 3, 2, 1};
 
 struct Lane {
-    const uint8_t* pg;
-    bool aligned;
-    uint64_t words, cursor;
     uint64_t bb;
     uint32_t left;
+    // the words ahead: lane l holds words l and 32 + l of the 64 from the
+    // cursor's group on, so a refill is two shuffles and the loads run 32
+    // words ahead of their use
+    uint32_t at;          // the cursor within the group, below 32
+    uint32_t w0, w1;
+    const uint8_t* next;  // the word that lane 0 loads next
+    uint64_t avail;       // words from the cursor on
+    bool aligned;
 
-    __device__ __forceinline__ uint32_t word(uint64_t i) const {
-        const uint8_t* p = pg + 4 * i;
+    // The word `lane` words past `next`; `off` words past the cursor.
+    __device__ __forceinline__ uint32_t word(uint32_t lane, uint32_t off) const {
+        if (off >= avail) return 0;
+        const uint8_t* p = next + 4 * lane;
         if (aligned) return __ldg(reinterpret_cast<const uint32_t*>(p));
         return static_cast<uint32_t>(__ldg(p)) | (static_cast<uint32_t>(__ldg(p + 1)) << 8) |
                (static_cast<uint32_t>(__ldg(p + 2)) << 16) |
                (static_cast<uint32_t>(__ldg(p + 3)) << 24);
+    }
+    // The first 32 of the page's n words are the lanes' first bits.
+    __device__ __forceinline__ void begin(const uint8_t* page, uint64_t n, uint32_t lane) {
+        next = page;
+        aligned = (reinterpret_cast<uintptr_t>(page) & 3) == 0;
+        avail = n;
+        at = 0;
+        left = 32;
+        bb = word(lane, lane);
+        avail -= 32;
+        next += 128;
+        w0 = word(lane, lane);
+        next += 128;
+        w1 = word(lane, 32 + lane);
+        next += 128;
     }
     __device__ __forceinline__ void consume(uint32_t n) {
         bb >>= n;
@@ -90,10 +137,11 @@ struct Lane {
         const bool need = left < 32;
         const unsigned m = __ballot_sync(0xffffffffu, need);
         const uint32_t rank = __popc(m & ((1u << lane) - 1));
-        const uint64_t avail = words - cursor;
-        const uint32_t want = __popc(m);
+        const uint32_t want = __popc(m), i = at + rank;
+        const uint32_t v0 = __shfl_sync(0xffffffffu, w0, i & 31);
+        const uint32_t v1 = __shfl_sync(0xffffffffu, w1, i & 31);
         if (need && rank < avail) {
-            bb |= static_cast<uint64_t>(word(cursor + rank)) << left;
+            bb |= static_cast<uint64_t>(i < 32 ? v0 : v1) << left;
             left += 32;
         }
         uint32_t ev = kNoEvent;
@@ -101,107 +149,116 @@ struct Lane {
             // the lane whose rank equals avail is the first that finds no word
             const unsigned short_lanes = __ballot_sync(0xffffffffu, need && rank >= avail);
             ev = 2 * (__ffs(short_lanes) - 1) + 1;
+            at += static_cast<uint32_t>(avail);
+            avail = 0;
+        } else {
+            at += want;
+            avail -= want;
         }
-        cursor += want < avail ? want : avail;
+        if (at >= 32) {
+            at -= 32;
+            w0 = w1;
+            w1 = word(lane, 32 - at + lane);
+            next += 128;
+        }
         return ev;
     }
 };
 
-// Table from code lengths (count/sorted symbols for the canonical path and a
-// kTabBits lookup table). Lane 0 computes the canonical codes; all lanes fill
-// the table. Returns false (all lanes) when the code is over-subscribed.
-__device__ __forceinline__ bool build_code(Tables& sm, const uint8_t* lens, uint32_t n,
-                                           uint16_t* tab, uint16_t* count, uint16_t* sym,
-                                           uint32_t tbits, int32_t* first_out,
-                                           int32_t* index_out, uint32_t lane) {
+// Table from code lengths (sorted symbols for the longer codes and a lookup
+// table of tbits bits), 32 symbols at a time: a symbol's place among those of
+// its length is its rank in the group (a match over the lanes) past the
+// earlier groups'. Returns false (all lanes) when the code is
+// over-subscribed.
+static __device__ __noinline__ bool build_code(Tables& sm, const uint8_t* lens, uint32_t n,
+                                           uint16_t* tab, uint16_t* sym, uint32_t tbits,
+                                           Tables::Long* big, uint32_t lane) {
+    const uint32_t lt = (1u << lane) - 1;
+    uint16_t* next = sm.u.b.next;    // per length: the next code,
+    uint16_t* place = sm.u.b.place;  // and the next place in sym
+    uint16_t* count = sm.count;
     __syncwarp();
-    bool ok = true;
-    if (lane == 0) {
-        uint16_t cnt[16];
-        for (int b = 0; b < 16; ++b) cnt[b] = 0;
-        for (uint32_t s = 0; s < n; ++s) cnt[lens[s]]++;
-        int leftk = 1;
-        for (int b = 1; b < 16; ++b) {
-            leftk <<= 1;
-            leftk -= cnt[b];
-            if (leftk < 0) ok = false;
-        }
-        uint16_t offs[16], next[16];
-        offs[1] = 0;
-        for (int b = 1; b < 15; ++b) offs[b + 1] = offs[b] + cnt[b];
-        uint32_t c = 0;
-        cnt[0] = 0;
-        for (int b = 1; b < 16; ++b) {
-            c = (c + cnt[b - 1]) << 1;
-            next[b] = static_cast<uint16_t>(c);
-        }
-        for (int b = 0; b < 16; ++b) count[b] = cnt[b];
-        // the canonical walk's first code and symbol index once it has passed
-        // the lengths the lookup table holds (they depend on the counts only)
-        int32_t f = 0, ix = 0;
-        for (uint32_t b = 1; b <= tbits; ++b) {
-            ix += cnt[b];
-            f = (f + cnt[b]) << 1;
-        }
-        *first_out = f;
-        *index_out = ix;
-        for (uint32_t s = 0; s < n; ++s) {
-            const uint32_t l = lens[s];
-            if (l && ok) {
-                sym[offs[l]++] = static_cast<uint16_t>(s);
-                sm.code[s] = next[l]++;
-            }
-        }
+    if (lane < 16) count[lane] = 0;
+    __syncwarp();
+    for (uint32_t s0 = 0; s0 < n; s0 += 32) {
+        const uint32_t l = s0 + lane < n ? lens[s0 + lane] : 0u;
+        const unsigned same = __match_any_sync(0xffffffffu, l);
+        if (l && (same >> lane) == 1u) count[l] = static_cast<uint16_t>(count[l] + __popc(same));
+        __syncwarp();
     }
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    // every lane walks the lengths; lane b keeps length b's first code and place
+    int leftk = 1;
+    bool ok = true;
+    uint32_t c = 0, at = 0, prev = 0;
+    for (uint32_t b = 1; b < 16; ++b) {
+        const uint32_t k = count[b];
+        leftk = (leftk << 1) - static_cast<int>(k);
+        ok = ok && leftk >= 0;
+        c = (c + prev) << 1;
+        if (lane == b) {
+            next[b] = static_cast<uint16_t>(c);
+            place[b] = static_cast<uint16_t>(at);
+        }
+        if (lane == b && b > kTabBits && big) {
+            // a valid code's limits fit: c + k is at most 2^b
+            const uint32_t end = (c + k) << (15 - b);
+            big->limit[b - kTabBits - 1] = static_cast<uint16_t>(end < 0xffff ? end : 0xffff);
+            big->from[b - kTabBits - 1] = static_cast<uint16_t>(c << (15 - b));
+            big->index[b - kTabBits - 1] = static_cast<uint16_t>(at);
+        }
+        at += k;
+        prev = k;
+    }
     if (!ok) return false;
     const uint32_t size = 1u << tbits;
     for (uint32_t i = lane; i < size; i += 32) tab[i] = 0;
     __syncwarp();
-    for (uint32_t s = lane; s < n; s += 32) {
-        const uint32_t l = lens[s];
-        if (l == 0 || l > tbits) continue;
-        const uint32_t rc = __brev(static_cast<uint32_t>(sm.code[s])) >> (32 - l);
-        const uint16_t e = static_cast<uint16_t>(s | (l << 9));
-        for (uint32_t i = rc; i < size; i += 1u << l) tab[i] = e;
+    for (uint32_t s0 = 0; s0 < n; s0 += 32) {
+        const uint32_t s = s0 + lane;
+        const uint32_t l = s < n ? lens[s] : 0u;
+        const unsigned same = __match_any_sync(0xffffffffu, l);
+        const uint32_t rank = __popc(same & lt);
+        const uint32_t code = next[l] + rank, to = place[l] + rank;  // unused for l = 0
+        __syncwarp();
+        if (l) {
+            sym[to] = static_cast<uint16_t>(s);
+            if ((same >> lane) == 1u) {
+                next[l] = static_cast<uint16_t>(code + 1);
+                place[l] = static_cast<uint16_t>(to + 1);
+            }
+            if (l <= tbits) {
+                const uint32_t rc = __brev(code) >> (32 - l);
+                const uint16_t e = static_cast<uint16_t>(s | (l << 9));
+                for (uint32_t i = rc; i < size; i += 1u << l) tab[i] = e;
+            }
+        }
+        __syncwarp();
     }
-    __syncwarp();
     return true;
 }
 
 // Decode a code from the low bits of bb: symbol and length, or false. Codes
-// of up to kTabBits bits come from the lookup table; longer ones continue the
-// canonical walk at length kTabBits + 1 from the state build_code stored (a
-// zero table entry means no shorter code matched, so the walk would not have
-// stopped earlier), with the code so far the first kTabBits bits in reading
-// order.
-__device__ __forceinline__ bool decode_sym(uint64_t bb, const uint16_t* tab, const uint16_t* count,
-                                           const uint16_t* sym, int32_t first0, int32_t index0,
-                                           uint32_t* s, uint32_t* len) {
+// of up to kTabBits bits come from the lookup table. A longer one (a few per
+// cent of the symbols, so most rounds have one in some lane) is read
+// left-aligned in 15 bits: canonical codes ascend with their length, so its
+// length is the first whose limit lies above it, five comparisons without a
+// loop.
+__device__ __forceinline__ bool decode_sym(uint64_t bb, const uint16_t* tab, const uint16_t* sym,
+                                           const Tables::Long& big, uint32_t* s, uint32_t* len) {
     const uint16_t e = tab[bb & ((1u << kTabBits) - 1)];
     if (e) {
         *s = e & 511;
         *len = e >> 9;
         return true;
     }
-    int code = static_cast<int>(
-                   __brev(static_cast<uint32_t>(bb) & ((1u << kTabBits) - 1)) >> (32 - kTabBits))
-               << 1;
-    int first = first0, index = index0;
-    for (int l = kTabBits + 1; l <= 15; ++l) {
-        code |= static_cast<int>((bb >> (l - 1)) & 1);
-        const int c = count[l];
-        if (code - c < first) {
-            *s = sym[index + (code - first)];
-            *len = static_cast<uint32_t>(l);
-            return true;
-        }
-        index += c;
-        first += c;
-        first <<= 1;
-        code <<= 1;
-    }
-    return false;
+    const uint32_t code = __brev(static_cast<uint32_t>(bb)) >> 17;
+    uint32_t k = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 5; ++j) k += code >= big.limit[j];
+    if (k == 5) return false;
+    *len = kTabBits + 1 + k;
+    *s = sym[big.index[k] + ((code - big.from[k]) >> (4 - k))];
+    return true;
 }
 
 // The first event of a round: op errors (phase 0, status in st) against the
@@ -214,22 +271,16 @@ __device__ __forceinline__ int first_event(bool err, int st, uint32_t refill_ev,
     return CUDEC_ERR_CORRUPT_INPUT;
 }
 
-// Copy [o, o + n) from o - d inside the page's output (d <= o), one lane,
-// in 16-byte windows: the aligned words holding the bytes, joined by funnel
-// shifts, then the widest stores the destination's alignment allows. The
-// first window is one read and one write in every lane (a distance under 16
-// is expanded to 16 bytes by lzw::period16), the rest a plain copy at
-// lzw::rest_distance(d). Every byte a window reads was written before it, by
-// this lane or earlier.
-__device__ __forceinline__ void page_copy(uint8_t* out, uint32_t o, uint32_t n, uint32_t d) {
-    uint8_t* D = out + o;
-    const uint32_t m0 = n < 16 ? n : 16u;
-    lzw::st16_global(D, lzw::period16(lzw::ld16_words(D - d, d < 16 ? d : m0), d), m0);
-    const uint32_t q = lzw::rest_distance(d);
-    for (uint32_t k = 16; k < n; k += 16) {
-        const uint32_t m = n - k < 16 ? n - k : 16u;
-        lzw::st16_global(D + k, lzw::ld16_words(D + k - q, m), m);
-    }
+// Execute the first n (at most 32) of the queued matches: their positions
+// ascend, and every other byte before the last one's end is written.
+__device__ __forceinline__ void flush_queue(uint8_t* out, Tables& sm, uint32_t n,
+                                            uint32_t lane) {
+    __syncwarp();
+    const bool mine = lane < n;
+    const uint32_t at = mine ? sm.u.q.at[lane] : 0u, len = mine ? sm.u.q.len[lane] : 0u;
+    const uint32_t off = mine ? sm.u.q.off[lane] : 0u;
+    const uint32_t b0 = __shfl_sync(0xffffffffu, at, 0);
+    lanes::match_rounds(out, mine, at, len, off, b0, sm.u.q.period, lane);
 }
 
 // Decode one page; every lane returns the same status and *written. Output
@@ -242,8 +293,11 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
     *written = 0;
     uint8_t* const out = dst;
     if (N % 4 != 0 || N / 4 < 32) return CUDEC_ERR_CORRUPT_INPUT;
-    Lane ln{pg, (reinterpret_cast<uintptr_t>(pg) & 3) == 0, N / 4, 32, 0, 32};
-    ln.bb = ln.word(lane);
+    Lane ln;
+    ln.begin(pg, N / 4, lane);
+    __syncwarp();
+    if (lane < 29) sm.base[lane] = kLBase[lane] | static_cast<uint32_t>(kLExtra[lane]) << 24;
+    sm.base[32 + lane] = kDBase[lane] | static_cast<uint32_t>(kDExtra[lane]) << 24;
     uint32_t pos = 0;
     const uint64_t room = cap;
     bool final = false;
@@ -281,7 +335,7 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
         uint32_t hlit = 288, hdist = 32;
         if (btype == 1) {
             for (uint32_t s = lane; s < 320; s += 32)
-                sm.lens[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : s < 288 ? 8 : 5;
+                sm.u.b.lens[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : s < 288 ? 8 : 5;
             __syncwarp();
         } else {
             const uint32_t h = __shfl_sync(0xffffffffu, static_cast<uint32_t>(ln.bb & 0x3FFF), 0);
@@ -291,23 +345,21 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
             if (lane == 0) ln.consume(14);
             if (ln.refill(lane) != kNoEvent) return CUDEC_ERR_CORRUPT_INPUT;
             if (hlit > 288 || hdist > 32) return CUDEC_ERR_CORRUPT_INPUT;
-            if (lane < 19) sm.plen[kPerm[lane]] = 0;
+            if (lane < 19) sm.u.b.plen[kPerm[lane]] = 0;
             __syncwarp();
             if (lane < hclen) {
-                sm.plen[kPerm[lane]] = static_cast<uint8_t>(ln.bb & 7);
+                sm.u.b.plen[kPerm[lane]] = static_cast<uint8_t>(ln.bb & 7);
                 ln.consume(3);
             }
             if (ln.refill(lane) != kNoEvent) return CUDEC_ERR_CORRUPT_INPUT;
             // precode: complete 7-bit table (its codes are at most 7 bits)
-            // (the precode's walk state is not used: its codes fit its table)
-            if (!build_code(sm, sm.plen, 19, sm.ptab, sm.lcount, sm.lsym, 7, &sm.lfirst,
-                            &sm.lindex, lane))
+            if (!build_code(sm, sm.u.b.plen, 19, sm.u.b.ptab, sm.lsym, 7, nullptr, lane))
                 return CUDEC_ERR_CORRUPT_INPUT;
             const uint32_t total = hlit + hdist;
             uint32_t have = 0;
             uint32_t prev_last = 0;  // the last length written so far
             while (have < total) {
-                const uint16_t e = sm.ptab[ln.bb & 127];
+                const uint16_t e = sm.u.b.ptab[ln.bb & 127];
                 const bool valid = e != 0;
                 const uint32_t sym = e & 511, clen = e >> 9;
                 uint32_t rep = 1, xb = 0, val = sym;
@@ -346,7 +398,7 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
                 if (v == 0xFFFFu) v = prev_last;
                 if (act && st == CUDEC_OK) {
                     ln.consume(clen + xb);
-                    for (uint32_t k = 0; k < rep; ++k) sm.lens[have + excl + k] = static_cast<uint8_t>(v);
+                    for (uint32_t k = 0; k < rep; ++k) sm.u.b.lens[have + excl + k] = static_cast<uint8_t>(v);
                 }
                 const uint32_t rev = ln.refill(lane);
                 const int s = first_event(st != CUDEC_OK, st, rev, lane);
@@ -357,17 +409,18 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
                 have += __shfl_sync(0xffffffffu, incl, last);
                 __syncwarp();
             }
-            if (sm.lens[256] == 0) return CUDEC_ERR_CORRUPT_INPUT;
+            if (sm.u.b.lens[256] == 0) return CUDEC_ERR_CORRUPT_INPUT;
         }
-        if (!build_code(sm, sm.lens, hlit, sm.ltab, sm.lcount, sm.lsym, kTabBits, &sm.lfirst,
-                        &sm.lindex, lane))
+        if (!build_code(sm, sm.u.b.lens, hlit, sm.ltab, sm.lsym, kTabBits, &sm.llong, lane))
             return CUDEC_ERR_CORRUPT_INPUT;
-        if (!build_code(sm, sm.lens + hlit, hdist, sm.dtab, sm.dcount, sm.dsym, kTabBits,
-                        &sm.dfirst, &sm.dindex, lane))
+        if (!build_code(sm, sm.u.b.lens + hlit, hdist, sm.dtab, sm.dsym, kTabBits, &sm.dlong,
+                        lane))
             return CUDEC_ERR_CORRUPT_INPUT;
         // ---- data rounds ----
         bool pend = false, eob = false;
         uint32_t ppos = 0, plen = 0;
+        uint32_t queued = 0;
+        __syncwarp();  // the queue takes the place of what built the tables
         for (;;) {
             const bool want_dist = pend;
             const bool want_lit = !pend && !eob;
@@ -377,9 +430,8 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
             // so the warp does not run the two in turn
             if (want_dist || want_lit) {
                 const bool dd = want_dist;
-                valid = decode_sym(ln.bb, dd ? sm.dtab : sm.ltab, dd ? sm.dcount : sm.lcount,
-                                   dd ? sm.dsym : sm.lsym, dd ? sm.dfirst : sm.lfirst,
-                                   dd ? sm.dindex : sm.lindex, &sym, &clen);
+                valid = decode_sym(ln.bb, dd ? sm.dtab : sm.ltab, dd ? sm.dsym : sm.lsym,
+                                   dd ? sm.dlong : sm.llong, &sym, &clen);
             }
             const unsigned eobm = __ballot_sync(0xffffffffu, want_lit && valid && sym == 256);
             const uint32_t e = eobm ? __ffs(eobm) - 1 : 32;
@@ -392,21 +444,17 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
             uint32_t L = 0, xb = 0, d = 0;
             int st = CUDEC_OK;
             if (act) {
-                if (!valid) {
+                if (!valid || (!want_dist && sym > 285)) {
                     st = CUDEC_ERR_CORRUPT_INPUT;
-                } else if (want_dist) {
-                    xb = kDExtra[sym];
-                    d = kDBase[sym] + (static_cast<uint32_t>(ln.bb >> clen) & ((1u << xb) - 1));
-                } else if (sym < 256) {
+                } else if (!want_dist && sym < 256) {
                     L = 1;
-                } else if (sym > 256) {
-                    if (sym > 285) {
-                        st = CUDEC_ERR_CORRUPT_INPUT;
-                    } else {
-                        xb = kLExtra[sym - 257];
-                        L = kLBase[sym - 257] +
-                            (static_cast<uint32_t>(ln.bb >> clen) & ((1u << xb) - 1));
-                    }
+                } else if (want_dist || sym > 256) {
+                    const uint32_t bx = sm.base[want_dist ? 32 + sym : sym - 257];
+                    xb = bx >> 24;
+                    const uint32_t v = (bx & 0xffffff) +
+                                       (static_cast<uint32_t>(ln.bb >> clen) & ((1u << xb) - 1));
+                    if (want_dist) d = v;
+                    else L = v;
                 }
             }
             uint32_t incl = L;
@@ -429,26 +477,16 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
             if (s != CUDEC_OK) return s;
             // literals of this round
             if (act && want_lit && sym < 256) out[p] = static_cast<uint8_t>(sym);
-            __syncwarp();
-            // copies whose distance arrived: frontier order by position
-            bool go = act && want_dist;
-            while (__any_sync(0xffffffffu, go)) {
-                uint32_t front = go ? ppos : 0xFFFFFFFFu;
-#pragma unroll
-                for (uint32_t k = 16; k; k >>= 1) {
-                    const uint32_t o = __shfl_xor_sync(0xffffffffu, front, k);
-                    front = o < front ? o : front;
-                }
-                if (go) {
-                    const uint32_t src_end = ppos - d + plen;
-                    const uint32_t need = src_end < ppos ? src_end : ppos;
-                    if (need <= front) {
-                        page_copy(out, ppos, plen, d);
-                        go = false;
-                    }
-                }
-                __syncwarp();
+            // matches whose distance arrived
+            const bool ready = act && want_dist;
+            const unsigned rm = __ballot_sync(0xffffffffu, ready);
+            if (ready) {
+                const uint32_t i = queued + __popc(rm & ((1u << lane) - 1));
+                sm.u.q.at[i] = ppos;
+                sm.u.q.len[i] = plen;
+                sm.u.q.off[i] = d;
             }
+            queued += __popc(rm);
             if (act && want_dist) pend = false;
             if (act && want_lit && sym > 256) {
                 pend = true;
@@ -457,10 +495,22 @@ __device__ __forceinline__ int decode_page(const uint8_t* pg, uint64_t N, uint8_
             }
             pos += __shfl_sync(0xffffffffu, incl, 31);
             if (e < 32) eob = true;
-            if (eob && !__any_sync(0xffffffffu, pend)) break;
+            const bool done = eob && !__any_sync(0xffffffffu, pend);
+            while (queued >= 32 || (done && queued)) {
+                const uint32_t n = queued < 32 ? queued : 32u;
+                flush_queue(out, sm, n, lane);
+                queued -= n;
+                if (lane < queued) {
+                    sm.u.q.at[lane] = sm.u.q.at[32 + lane];
+                    sm.u.q.len[lane] = sm.u.q.len[32 + lane];
+                    sm.u.q.off[lane] = sm.u.q.off[32 + lane];
+                }
+                __syncwarp();
+            }
+            if (done) break;
         }
     }
-    if (ln.cursor != ln.words) return CUDEC_ERR_CORRUPT_INPUT;
+    if (ln.avail != 0) return CUDEC_ERR_CORRUPT_INPUT;
     __syncwarp();
     *written = pos;
     return CUDEC_OK;

@@ -5,8 +5,9 @@ collectives and barriers (a deadlock, lanes at different collectives, or
 threads that disagree on the result fail the run), in an order drawn from a
 seed. The sizes are those where the decoders change their way: LZ4 and Snappy
 chunks of one tile and of several at each width of the CTA, batches cut by
-long tokens, tiles that few tokens settle. Statuses, bytes and untouched
-memory around them equal the oracle's; the mutants cover the early ends.
+long tokens, tiles that few tokens settle; short GDeflate pages and full ones.
+Statuses, bytes and untouched memory around them equal the oracle's; the
+mutants cover the early ends.
 """
 import ctypes
 import os
@@ -51,6 +52,15 @@ def lz():
     return call
 
 
+@pytest.fixture(scope="module")
+def gdeflate():
+    lib = _build("gdeflate_emul")
+    lib.gdeflate_emulate.argtypes = [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p,
+                                     ctypes.c_uint64, ctypes.c_uint64,
+                                     ctypes.POINTER(ctypes.c_uint64)]
+    return lib.gdeflate_emulate
+
+
 def check(run, want, comp, cap, seed=0, skew=0, label=None):
     src = np.zeros(len(comp) + 64 + skew, dtype=np.uint8)
     src[32 + skew:32 + skew + len(comp)] = np.frombuffer(comp, dtype=np.uint8)
@@ -82,7 +92,7 @@ def mutate(rng, comp):
 
 def contents(size):
     rng = random.Random(size)
-    yield W.generate([max(size, 1)], W.lz_params(), seeds=[size])[0][:size].tobytes()
+    yield W.generate([max(size, 1)], W.zstd_params(), seeds=[size])[0][:size].tobytes()
     yield bytes(size)
     yield rng.randbytes(size)
     yield (b"the quick brown fox jumps over the lazy dog; " * (size // 45 + 1))[:size]
@@ -114,3 +124,18 @@ def test_lz(lz, size, threads):
             for m in range(4 if size < 6000 else 1):
                 check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2, m, 0,
                       (size, k, fmt, m))
+
+
+@pytest.mark.parametrize("size", [0, 1, 63, 3000, 20000, 65536])
+def test_gdeflate(gdeflate, size):
+    rng = random.Random(size)
+    pages = list(contents(size))
+    pages.append(W.generate([max(size, 1)], W.gdeflate_params(0.8), seeds=[9])[0][:size].tobytes())
+    for k, data in enumerate(pages):
+        for level in (1, 12):
+            f = W.gdeflate_compress(data, level)
+            check(gdeflate, oracle.gdeflate_decode, f, size, k, (5 * k + level) % 16,
+                  (size, k, level))
+            for m in range(3 if size > 5000 else 12):
+                check(gdeflate, oracle.gdeflate_decode, mutate(rng, f), size - (m % 2) * size // 2,
+                      m, 0, (size, k, level, m))
