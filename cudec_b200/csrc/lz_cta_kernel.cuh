@@ -92,7 +92,7 @@ struct Width {
     static constexpr uint32_t kWarps = T / 32;
     static constexpr uint32_t kTile = T * kReg;  // positions per tile: a region per thread
     static constexpr uint32_t kInBytes = (kTile + kLook + 32 + 15) / 16 * 16;  // staged input
-    static constexpr uint32_t kUnroll = T == 128 ? 4 : 2;      // sectors in flight per warp
+    static constexpr uint32_t kUnroll = T == 128 ? 3 : 2;      // sectors in flight per warp
     static constexpr uint32_t kPart = 32 * kWarps * kUnroll;  // output bytes between barriers
     // resident CTAs per SM that the registers are compiled for
     static constexpr int kPerSm = T == 128 ? 7 : T == 256 ? 3 : 1;
@@ -818,17 +818,14 @@ struct Chunk {
                 uint32_t a[kUnroll], m[kUnroll];
                 LZG_UNROLL
                 for (uint32_t j = 0; j < kUnroll; ++j) {
-                    const uint32_t y = 32 * (k + j * kWarps) + lane;
-                    const bool in_range = y - lo < hi - lo;
                     a[j] = m[j] = 0;
-                    if (in_range && !src[j].lit) m[j] = wb[src[j].at];
-                    if (in_range && src[j].lit) a[j] = in[src[j].at];
+                    if (src[j].ok && !src[j].lit) m[j] = wb[src[j].at];
+                    if (src[j].ok && src[j].lit) a[j] = in[src[j].at];
                 }
+                uint8_t* y = wb + 32 * k + lane;
                 LZG_UNROLL
-                for (uint32_t j = 0; j < kUnroll; ++j) {
-                    const uint32_t y = 32 * (k + j * kWarps) + lane;
-                    if (y - lo < hi - lo) wb[y] = static_cast<uint8_t>(src[j].lit ? a[j] : m[j]);
-                }
+                for (uint32_t j = 0; j < kUnroll; ++j)
+                    if (src[j].ok) y[32 * j * kWarps] = static_cast<uint8_t>(a[j] | m[j]);
             });
         }
     }

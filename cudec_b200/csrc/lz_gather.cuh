@@ -82,6 +82,7 @@ CDB_HD void map_token(Sector* map, uint32_t i, uint32_t y0, uint32_t y1, uint32_
 struct Source {
     int32_t at;
     bool lit;
+    bool ok;  // the byte is one of the batch's
 };
 
 #if defined(__CUDA_ARCH__)
@@ -95,8 +96,8 @@ struct Source {
 // A source inside the window is followed through the map, past whole periods
 // of an overlapping match, so each match costs one hop at most (matches are
 // shorter than 2^12 bytes, see small_mod; offsets are below 2^31). The loads
-// of all N run together; the bytes that need another hop (0.13 per byte on
-// chunks of 12-byte tokens) go on in a loop that most groups skip.
+// of all N run together; the bytes that need another hop go on in a loop
+// that most groups skip.
 template <uint32_t N, uint32_t kRecs>
 CDB_HD void sources(const Sector* map, const Rec* rec, uint32_t k, uint32_t step, uint32_t lane,
                     uint32_t lo, uint32_t hi, uint32_t W, Source (&src)[N]) {
@@ -119,8 +120,8 @@ CDB_HD void sources(const Sector* map, const Rec* rec, uint32_t k, uint32_t step
         src[j].lit = static_cast<int32_t>(m) < 0;
         src[j].at = static_cast<int32_t>(src[j].lit ? x + W + static_cast<uint32_t>(src[j].at)
                                                     : x - off[j]);
-        const bool more = !src[j].lit && (m >= off[j] || off[j] <= x - lo) && x - lo < hi - lo;
-        any = any || more;
+        src[j].ok = x - lo < hi - lo;
+        any = any || (src[j].ok && !src[j].lit && (m >= off[j] || off[j] <= x - lo));
     }
 #if CDB_DEVICE_CODE
     if (!__any_sync(0xffffffffu, any)) return;
@@ -130,20 +131,21 @@ CDB_HD void sources(const Sector* map, const Rec* rec, uint32_t k, uint32_t step
     LZG_UNROLL
     for (uint32_t j = 0; j < N; ++j) {
         uint32_t x = 32 * (k + j * step) + lane;
-        if (src[j].lit || x - lo >= hi - lo) continue;
+        if (src[j].lit || !src[j].ok) continue;
         uint32_t end = le[j], by = off[j];
         for (;;) {
             const uint32_t m = x + W - end;
             if (m >= by) by += m - small_mod(m, by);
             if (by > x - lo) {
-                src[j] = Source{static_cast<int32_t>(x - by), false};
+                src[j].at = static_cast<int32_t>(x - by);
                 break;
             }
             x -= by;
             const Sector sc = map[x >> 5];
             const Rec r = rec[sc.before + pop32(sc.starts & (0xffffffffu >> (31 - (x & 31)))) - 1];
             if (static_cast<int32_t>(x + W - r.le) < 0) {
-                src[j] = Source{static_cast<int32_t>(x + W + r.dl), true};
+                src[j].at = static_cast<int32_t>(x + W + r.dl);
+                src[j].lit = true;
                 break;
             }
             end = r.le;

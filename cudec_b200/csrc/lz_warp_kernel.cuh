@@ -639,18 +639,6 @@ __device__ __noinline__ Walk walk_group(const uint8_t* win, uint32_t gb, uint32_
     return Walk{myr, myo, cnt};
 }
 
-// Store m (1..16) bytes of v at global p (16-byte store when aligned and whole).
-__device__ __forceinline__ void st16_global(uint8_t* p, const uint4& v, uint32_t m) {
-    if (m == 16 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        *reinterpret_cast<uint4*>(p) = v;
-        return;
-    }
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (uint32_t j = 0; j < 16; ++j)
-        if (j < m) p[j] = static_cast<uint8_t>(w[j >> 2] >> ((j & 3) * 8));
-}
-
 // The whole warp copies n input bytes at g + src to dst + o (no overlap):
 // destination-aligned 16-byte stores, four in flight per lane.
 __device__ __forceinline__ void coop_literal(uint8_t* dst, uint64_t o, const uint8_t* src, uint64_t n,

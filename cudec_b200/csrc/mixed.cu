@@ -10,12 +10,11 @@
 //     chunks start first and the tail of the launch is short chunks;
 //   * a work counter: every warp of the persistent grid takes the next chunk
 //     of that order with one atomic add (work stealing), whatever its format;
-//   * warps per chunk by size bucket: LZ4 and Snappy chunks of the buckets
-//     set to a whole CTA go first in the order (largest first among them)
-//     and are taken, one chunk per CTA, by the CTA-per-chunk decoder
-//     (lz_cta_kernel.cuh) in a second persistent grid that runs beside the
-//     warp grid; the warp grid starts after them;
-//   * per-warp Zstd literal slots;
+//   * three persistent grids side by side: Zstd frames go first in the order
+//     and are taken, one frame per CTA, by the CTA decoder of zstd_frame.cuh
+//     (a literal slot per CTA); then LZ4 and Snappy chunks of the size buckets
+//     set to a whole CTA, one chunk per CTA of lz_cta_kernel.cuh; the warp
+//     grid starts after them;
 //   * the decode shape per size bucket (warps per chunk; for one warp, the
 //     parse window, input lookahead and ring batch) chosen by
 //     cudec_mixed_plan_tune, which times candidate shapes on the caller's
@@ -29,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <new>
@@ -50,17 +50,18 @@ constexpr uint32_t kWarps = 4;
 constexpr uint32_t kThreads = 32 * kWarps;
 constexpr uint32_t kMaxOf(uint32_t a, uint32_t b) { return a > b ? a : b; }
 constexpr uint32_t kWarpSmem =
-    kMaxOf(kMaxOf(lzw::kWarpSmem, static_cast<uint32_t>(sizeof(zstd::WarpSmem))),
-           static_cast<uint32_t>(sizeof(gdf::Tables)));
+    kMaxOf(lzw::kWarpSmem, static_cast<uint32_t>(sizeof(gdf::Tables)));
 constexpr uint32_t kSmem = kWarps * kWarpSmem;
 constexpr int kBuckets = CUDEC_MIXED_BUCKETS;
 constexpr int kSizeClasses = 64;  // floor(log2(capacity)) classes for the order
-constexpr int kClasses = 2 * kSizeClasses;  // CTA-decoded chunks: the upper half
+// Order classes: one-warp chunks, LZ4 / Snappy chunks of a CTA, Zstd frames.
+constexpr int kClasses = 3 * kSizeClasses;
 // The shape value that names the CTA decoder (its own width is lzc::kThreads).
 constexpr uint32_t kCtaWarps = CUDEC_MIXED_CTA_WARPS;
-// Resident CTAs per SM of the CTA grid, at most: they leave room for the warp
-// grid that decodes beside it.
-constexpr int kCtaPerSmMax = 5;
+// Resident CTAs per SM, at most, of the two CTA grids: they share the SMs with
+// each other and with the warp grid. The Zstd grid's limit is its kernel's own;
+// the LZ grid leaves room for the warp grid.
+constexpr int kCtaPerSmMax = 5, kZstdPerSmMax = 4;
 constexpr uint32_t kCtaSmem = kMaxOf(static_cast<uint32_t>(sizeof(lzc::Shm<lzc::Lz4F>)),
                                      static_cast<uint32_t>(sizeof(lzc::Shm<lzc::SnappyF>)));
 static_assert(kWarpSmem % 16 == 0, "per-warp regions stay 16-byte aligned");
@@ -76,12 +77,12 @@ __device__ __forceinline__ int size_class(uint64_t cap) {
     return cap ? 63 - __clzll(static_cast<long long>(cap)) : 0;
 }
 
-// The order class of chunk i: its size class, in the upper half when its
-// bucket decodes LZ4 / Snappy with a whole CTA (bit b of cta_buckets).
+// The order class of chunk i: its size class in its group (LZ4 / Snappy chunks
+// are a CTA's where bit b of cta_buckets is set for their bucket b).
 __device__ __forceinline__ int order_class(uint64_t cap, uint8_t fmt, uint32_t cta_buckets) {
     const bool cta = (fmt == CUDEC_FORMAT_LZ4 || fmt == CUDEC_FORMAT_SNAPPY) &&
                      ((cta_buckets >> size_bucket(cap)) & 1u);
-    return size_class(cap) + (cta ? kSizeClasses : 0);
+    return size_class(cap) + (fmt == CUDEC_FORMAT_ZSTD ? 2 * kSizeClasses : cta ? kSizeClasses : 0);
 }
 
 struct Args {
@@ -95,17 +96,15 @@ struct Args {
     const uint32_t* order;
     unsigned long long* counter;
     const unsigned long long* first;  // order index of the warp grid's first chunk
-    uint8_t* zstd_slots;
     lzw::Tune tune[kBuckets];
 };
 
-// Control block in device memory: the warp grid's and the CTA grid's work
-// counters, class counts and cursors, and the number of CTA-decoded chunks
-// (they occupy order[0, ncta)).
+// Control block in device memory: the grids' work counters, the order index
+// past the Zstd frames (order[0, nzstd)) and past the CTA-decoded LZ4 / Snappy
+// chunks (order[nzstd, ncta)), class counts and cursors.
 struct Ctrl {
-    unsigned long long counter;
-    unsigned long long cta_counter;
-    unsigned long long ncta;
+    unsigned long long counter, cta_counter, zstd_counter;
+    unsigned long long nzstd, ncta;
     unsigned long long counts[kClasses];
     unsigned long long cursor[kClasses];
 };
@@ -123,14 +122,15 @@ __global__ void order_count(const size_t* caps, const uint8_t* formats, size_t n
         if (h[i]) atomicAdd(&ctrl->counts[i], static_cast<unsigned long long>(h[i]));
 }
 
-// Start of each class in the order, largest class first, the CTA-decoded
-// half before the rest (one thread).
+// Start of each class in the order, largest class first within its group, the
+// groups in turn (one thread).
 __global__ void order_scan(Ctrl* ctrl) {
     if (threadIdx.x != 0) return;
     unsigned long long at = 0;
     for (int c = kClasses - 1; c >= 0; --c) {
         ctrl->cursor[c] = at;
         at += ctrl->counts[c];
+        if (c == 2 * kSizeClasses) ctrl->nzstd = at;
         if (c == kSizeClasses) ctrl->ncta = at;
     }
 }
@@ -145,8 +145,8 @@ __global__ void order_place(const size_t* caps, const uint8_t* formats, size_t n
     }
 }
 
-// The CTA grid: each CTA takes the next chunk of order[0, ncta) and decodes
-// it with the CTA-per-chunk decoder of its format.
+// The CTA grids: each CTA takes the next chunk of its part of the order and
+// decodes it.
 struct CtaArgs {
     const void* const* src;
     const size_t* sizes;
@@ -156,39 +156,68 @@ struct CtaArgs {
     cudec_chunk_result* results;
     const uint32_t* order;
     Ctrl* ctrl;
+    uint8_t* zstd_slots;
 };
+
+// The next order index of [from, to), or ~0: the same for every thread.
+__device__ __forceinline__ unsigned long long claim(unsigned long long* counter,
+                                                    unsigned long long from,
+                                                    unsigned long long to) {
+    __shared__ unsigned long long mine;
+    if (threadIdx.x == 0) mine = atomicAdd(counter, 1ull);
+    __syncthreads();
+    const unsigned long long idx = from + mine;
+    __syncthreads();  // read by every thread before the next claim is written
+    return idx < to ? idx : ~0ull;
+}
+
+__device__ __forceinline__ void record(cudec_chunk_result* r, int st, uint64_t written) {
+    if (threadIdx.x == 0) {
+        r->status = st;
+        r->reserved = 0;
+        r->bytes_written = st == CUDEC_OK ? written : 0;
+    }
+    __syncthreads();  // the next chunk reuses the shared state
+}
+
+template <class F>
+__device__ __noinline__ int mixed_cta_lz(const uint8_t* src, uint64_t S, uint8_t* dst,
+                                         uint64_t cap, uint64_t* written) {
+    extern __shared__ __align__(16) uint8_t cta_smem[];
+    lzc::Chunk<F> ch{*reinterpret_cast<lzc::Shm<F>*>(cta_smem), src, S, dst, cap, 0};
+    return ch.run(written);
+}
 
 __global__ void __launch_bounds__(lzc::kThreads, lzc::Width<lzc::kThreads>::kPerSm)
     mixed_cta_kernel(CtaArgs a) {
-    extern __shared__ __align__(16) uint8_t cta_smem[];
-    __shared__ unsigned long long claim;
-    const unsigned long long ncta = a.ctrl->ncta;
+    const unsigned long long from = a.ctrl->nzstd, to = a.ctrl->ncta;
     for (;;) {
-        if (threadIdx.x == 0) claim = atomicAdd(&a.ctrl->cta_counter, 1ull);
-        __syncthreads();
-        const unsigned long long idx = claim;
-        __syncthreads();  // read by every thread before the next claim is written
-        if (idx >= ncta) break;
+        const unsigned long long idx = claim(&a.ctrl->cta_counter, from, to);
+        if (idx == ~0ull) break;
         const uint32_t c = a.order[idx];
         const uint8_t* src = static_cast<const uint8_t*>(a.src[c]);
         uint8_t* dst = static_cast<uint8_t*>(a.dst[c]);
         uint64_t written = 0;
-        int st;
-        if (a.formats[c] == CUDEC_FORMAT_LZ4) {
-            lzc::Chunk<lzc::Lz4F> ch{*reinterpret_cast<lzc::Shm<lzc::Lz4F>*>(cta_smem), src,
-                                     a.sizes[c], dst, a.caps[c], 0};
-            st = ch.run(&written);
-        } else {
-            lzc::Chunk<lzc::SnappyF> ch{*reinterpret_cast<lzc::Shm<lzc::SnappyF>*>(cta_smem),
-                                        src, a.sizes[c], dst, a.caps[c], 0};
-            st = ch.run(&written);
-        }
-        if (threadIdx.x == 0) {
-            a.results[c].status = st;
-            a.results[c].reserved = 0;
-            a.results[c].bytes_written = st == CUDEC_OK ? written : 0;
-        }
-        __syncthreads();  // the next chunk reuses the shared state
+        const int st = a.formats[c] == CUDEC_FORMAT_LZ4
+                           ? mixed_cta_lz<lzc::Lz4F>(src, a.sizes[c], dst, a.caps[c], &written)
+                           : mixed_cta_lz<lzc::SnappyF>(src, a.sizes[c], dst, a.caps[c], &written);
+        record(&a.results[c], st, written);
+    }
+}
+
+__global__ void __launch_bounds__(zstd::kTeam, kZstdPerSmMax) mixed_zstd_kernel(CtaArgs a) {
+    __shared__ zstd::TeamSmem smem;
+    uint8_t* slot = a.zstd_slots + static_cast<size_t>(blockIdx.x) * zstd::kLitSlot;
+    const unsigned long long to = a.ctrl->nzstd;
+    for (;;) {
+        const unsigned long long idx = claim(&a.ctrl->zstd_counter, 0, to);
+        if (idx == ~0ull) break;
+        const uint32_t c = a.order[idx];
+        uint64_t written = 0;
+        const int st = zstd::decode_frame(static_cast<const uint8_t*>(a.src[c]), a.sizes[c],
+                                          static_cast<uint8_t*>(a.dst[c]), a.caps[c], smem, slot,
+                                          &written);
+        record(&a.results[c], st, written);
     }
 }
 
@@ -199,13 +228,6 @@ __device__ __noinline__ int mixed_lz(const uint8_t* src, uint64_t S, uint8_t* ds
                                      uint8_t* base, lzw::Tune tn, uint32_t lane,
                                      uint64_t* written) {
     return lzw::decode_chunk<F>(src, S, dst, cap, base, base + lzw::kRing, tn, lane, written);
-}
-
-__device__ __noinline__ int mixed_zstd(const uint8_t* src, uint64_t S, uint8_t* dst, uint64_t cap,
-                                       uint8_t* base, uint8_t* litbuf, uint32_t lane,
-                                       uint64_t* written) {
-    return zstd::decode_frame(src, S, dst, cap, *reinterpret_cast<zstd::WarpSmem*>(base), litbuf,
-                              lane, written);
 }
 
 __device__ __noinline__ int mixed_gdeflate(const uint8_t* src, uint64_t S, uint8_t* dst,
@@ -219,8 +241,6 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Args a) {
     extern __shared__ __align__(16) uint8_t mixed_smem[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint8_t* base = mixed_smem + warp * kWarpSmem;
-    const size_t gw = static_cast<size_t>(blockIdx.x) * kWarps + warp;
-    uint8_t* litbuf = a.zstd_slots + gw * zstd::kLitSlot;
     for (;;) {
         unsigned long long idx = 0;
         if (lane == 0) idx = *a.first + atomicAdd(a.counter, 1ull);
@@ -244,9 +264,6 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Args a) {
             case CUDEC_FORMAT_GDEFLATE:
                 st = mixed_gdeflate(src, S, dst, cap, base, lane, &written);
                 break;
-            case CUDEC_FORMAT_ZSTD:
-                st = mixed_zstd(src, S, dst, cap, base, litbuf, lane, &written);
-                break;
             default:
                 st = CUDEC_ERR_UNSUPPORTED;
                 break;
@@ -264,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Args a) {
 // below 16 KiB, a whole CTA from 16 KiB up (what the tuner picks on B200
 // over 100,000 uneven LZ4 + Snappy chunks, run after run: small chunks keep
 // the warp grid busy beside the CTA grid, and the CTA decoder's parallel
-// parse wins from 16 KiB up); Zstd and GDeflate chunks are one warp's.
+// parse wins from 16 KiB up); a GDeflate page is one warp's.
 constexpr uint32_t kDefaultWpc[kBuckets] = {1, 1, kCtaWarps, kCtaWarps, kCtaWarps, kCtaWarps};
 
 struct Key {
@@ -287,12 +304,14 @@ struct Key {
 struct cudec_mixed_plan {
     int dev = -1;
     unsigned grid = 0;      // warp grid: resident CTAs x SMs
-    unsigned cta_grid = 0;  // CTA grid: resident CTAs x SMs
+    unsigned cta_grid = 0;  // LZ CTA grid: resident CTAs x SMs
+    unsigned zstd_grid = 0;  // Zstd grid, likewise
     int sms = 0;
     cdb::DevBuf ctrl, order, slots;
-    cudaStream_t s = nullptr, s2 = nullptr;  // s2: the CTA grid beside the warp grid
+    cudaStream_t s = nullptr, s2 = nullptr, s3 = nullptr;  // s2, s3: the CTA grids beside
+                                                           // the warp grid
     cudaEvent_t ev_in = nullptr, ev_out = nullptr, t0 = nullptr, t1 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join3 = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cdb::mixed::Key key{};
@@ -315,11 +334,13 @@ struct cudec_mixed_plan {
     ~cudec_mixed_plan() {
         if (s) (void)cudaStreamSynchronize(s);
         if (s2) (void)cudaStreamSynchronize(s2);
+        if (s3) (void)cudaStreamSynchronize(s3);
         drop_graph();
-        for (cudaEvent_t e : {ev_in, ev_out, t0, t1, ev_fork, ev_join})
+        for (cudaEvent_t e : {ev_in, ev_out, t0, t1, ev_fork, ev_join, ev_join3})
             if (e) (void)cudaEventDestroy(e);
         if (s) (void)cudaStreamDestroy(s);
         if (s2) (void)cudaStreamDestroy(s2);
+        if (s3) (void)cudaStreamDestroy(s3);
     }
 };
 
@@ -349,7 +370,6 @@ Args make_args(cudec_mixed_plan* p, const Key& k) {
     a.order = static_cast<const uint32_t*>(p->order.p);
     a.counter = &static_cast<Ctrl*>(p->ctrl.p)->counter;
     a.first = &static_cast<Ctrl*>(p->ctrl.p)->ncta;
-    a.zstd_slots = static_cast<uint8_t*>(p->slots.p);
     for (int b = 0; b < cdb::mixed::kBuckets; ++b) a.tune[b] = p->tune[b];
     return a;
 }
@@ -360,7 +380,7 @@ Args make_args(cudec_mixed_plan* p, const Key& k) {
 cdb::mixed::CtaArgs make_cta_args(cudec_mixed_plan* p, const Key& k) {
     return cdb::mixed::CtaArgs{k.src, k.sizes, k.dst, k.caps, k.formats, k.results,
                                static_cast<const uint32_t*>(p->order.p),
-                               static_cast<Ctrl*>(p->ctrl.p)};
+                               static_cast<Ctrl*>(p->ctrl.p), static_cast<uint8_t*>(p->slots.p)};
 }
 
 cudaError_t enqueue(cudec_mixed_plan* p, const Key& k, cudaStream_t s) {
@@ -374,25 +394,30 @@ cudaError_t enqueue(cudec_mixed_plan* p, const Key& k, cudaStream_t s) {
     cdb::mixed::order_scan<<<1, 32, 0, s>>>(ctrl);
     cdb::mixed::order_place<<<blocks, 256, 0, s>>>(k.caps, k.formats, k.n, cb, ctrl,
                                                     static_cast<uint32_t*>(p->order.p));
-    if (cb) {
-        // the CTA grid beside the warp grid: forked to the plan's second
-        // stream after the order, joined back before the end
-        e = cudaEventRecord(p->ev_fork, s);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(p->s2, p->ev_fork, 0);
-        if (e != cudaSuccess) return e;
-        const unsigned cg = static_cast<unsigned>(std::min<size_t>(k.n, p->cta_grid));
-        cdb::mixed::mixed_cta_kernel<<<cg, cdb::lzc::kThreads, cdb::mixed::kCtaSmem, p->s2>>>(
-            make_cta_args(p, k));
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaEventRecord(p->ev_join, p->s2);
-        if (e != cudaSuccess) return e;
-    }
+    // the CTA grids beside the warp grid: forked to the plan's other streams
+    // after the order, joined back before the end
+    e = cudaEventRecord(p->ev_fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(p->s3, p->ev_fork, 0);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(p->s2, p->ev_fork, 0);
+    if (e != cudaSuccess) return e;
+    const unsigned zg = static_cast<unsigned>(std::min<size_t>(k.n, p->zstd_grid));
+    cdb::mixed::mixed_zstd_kernel<<<zg, cdb::zstd::kTeam, 0, p->s3>>>(make_cta_args(p, k));
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaEventRecord(p->ev_join3, p->s3);
+    if (e != cudaSuccess) return e;
+    const unsigned cg = static_cast<unsigned>(std::min<size_t>(k.n, p->cta_grid));
+    cdb::mixed::mixed_cta_kernel<<<cg, cdb::lzc::kThreads, cdb::mixed::kCtaSmem, p->s2>>>(
+        make_cta_args(p, k));
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaEventRecord(p->ev_join, p->s2);
+    if (e != cudaSuccess) return e;
     const size_t ctas = (k.n + cdb::mixed::kWarps - 1) / cdb::mixed::kWarps;
     const unsigned grid = static_cast<unsigned>(std::min<size_t>(ctas, p->grid));
     cdb::mixed::mixed_kernel<<<grid, cdb::mixed::kThreads, cdb::mixed::kSmem, s>>>(
         make_args(p, k));
     e = cudaGetLastError();
-    if (e == cudaSuccess && cb) e = cudaStreamWaitEvent(s, p->ev_join, 0);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, p->ev_join, 0);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, p->ev_join3, 0);
     return e;
 }
 
@@ -463,11 +488,18 @@ cudec_status cudec_mixed_plan_create(cudec_mixed_plan** out_plan) {
     if (cta_per_sm > cdb::mixed::kCtaPerSmMax) cta_per_sm = cdb::mixed::kCtaPerSmMax;
     if (ok) p->cta_grid = static_cast<unsigned>(p->sms * cta_per_sm);
     ok = ok && p->ctrl.ensure(sizeof(Ctrl)) == cudaSuccess;
-    ok = ok && p->slots.ensure(static_cast<size_t>(p->grid) * cdb::mixed::kWarps *
-                               cdb::zstd::kLitSlot) == cudaSuccess;
+    int zstd_per_sm = 0;
+    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                   &zstd_per_sm, cdb::mixed::mixed_zstd_kernel, cdb::zstd::kTeam, 0) == cudaSuccess;
+    ok = ok && zstd_per_sm > 0;
+    if (zstd_per_sm > cdb::mixed::kZstdPerSmMax) zstd_per_sm = cdb::mixed::kZstdPerSmMax;
+    if (ok) p->zstd_grid = static_cast<unsigned>(p->sms * zstd_per_sm);
+    ok = ok && p->slots.ensure(static_cast<size_t>(p->zstd_grid) * cdb::zstd::kLitSlot) ==
+                   cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&p->s, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&p->s2, cudaStreamNonBlocking) == cudaSuccess;
-    for (cudaEvent_t* e : {&p->ev_in, &p->ev_out, &p->ev_fork, &p->ev_join})
+    ok = ok && cudaStreamCreateWithFlags(&p->s3, cudaStreamNonBlocking) == cudaSuccess;
+    for (cudaEvent_t* e : {&p->ev_in, &p->ev_out, &p->ev_fork, &p->ev_join, &p->ev_join3})
         ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
     for (cudaEvent_t* e : {&p->t0, &p->t1}) ok = ok && cudaEventCreate(e) == cudaSuccess;
     if (!ok) {
@@ -547,8 +579,13 @@ cudec_status cudec_mixed_plan_tune(cudec_mixed_plan* plan, const void* const* d_
         cudaMemcpy(fmts.data(), d_formats, chunk_count, cudaMemcpyDeviceToHost) != cudaSuccess)
         return CUDEC_ERR_CUDA;
     std::vector<std::vector<uint32_t>> members(cdb::mixed::kBuckets), lz(cdb::mixed::kBuckets);
+    std::vector<uint32_t> zs;
     for (size_t i = 0; i < chunk_count; ++i) {
         const int bk = cdb::mixed::size_bucket(caps[i]);
+        if (fmts[i] == CUDEC_FORMAT_ZSTD) {  // always a CTA's: nothing to choose
+            zs.push_back(static_cast<uint32_t>(i));
+            continue;
+        }
         members[bk].push_back(static_cast<uint32_t>(i));
         if (fmts[i] == CUDEC_FORMAT_LZ4 || fmts[i] == CUDEC_FORMAT_SNAPPY)
             lz[bk].push_back(static_cast<uint32_t>(i));
@@ -567,16 +604,19 @@ cudec_status cudec_mixed_plan_tune(cudec_mixed_plan* plan, const void* const* d_
     const Key whole{d_src_ptrs, d_src_sizes, d_dst_ptrs, d_dst_capacities,
                     d_formats, chunk_count, d_results};
     Ctrl* ctrl = static_cast<Ctrl*>(plan->ctrl.p);
-    constexpr size_t kCounters = 2 * sizeof(unsigned long long);  // counter, cta_counter
+    constexpr size_t kCounters = 3 * sizeof(unsigned long long);
     // Best of two device-timed runs of `launch` on the plan's stream (after
-    // resetting the work counters and publishing the CTA grid's chunk
-    // count; every copy is on that stream, ordered with the launches).
-    auto timed = [&](auto launch, unsigned long long ncta, float* out) -> bool {
+    // resetting the work counters and publishing the CTA grids' parts of the
+    // order; every copy is on that stream, ordered with the launches).
+    auto timed = [&](auto launch, unsigned long long nzstd, unsigned long long ncta,
+                     float* out) -> bool {
         float ms_min = 0.f;
         for (int rep = 0; rep < 2; ++rep) {
             bool ok = cudaMemsetAsync(ctrl, 0, kCounters, plan->s) == cudaSuccess;
-            const unsigned long long h_ncta = ncta;  // pageable: staged before the call returns
-            ok = ok && cudaMemcpyAsync(&ctrl->ncta, &h_ncta, sizeof(h_ncta),
+            // pageable: staged before the call returns
+            const unsigned long long parts[2] = {nzstd, ncta};
+            static_assert(offsetof(Ctrl, ncta) == offsetof(Ctrl, nzstd) + sizeof(parts[0]));
+            ok = ok && cudaMemcpyAsync(&ctrl->nzstd, parts, sizeof(parts),
                                        cudaMemcpyHostToDevice, plan->s) == cudaSuccess;
             ok = ok && cudaEventRecord(plan->t0, plan->s) == cudaSuccess;
             launch();
@@ -608,7 +648,7 @@ cudec_status cudec_mixed_plan_tune(cudec_mixed_plan* plan, const void* const* d_
             if (!timed([&] {
                     cdb::mixed::mixed_kernel<<<plan->grid, cdb::mixed::kThreads,
                                                cdb::mixed::kSmem, plan->s>>>(a);
-                }, 0, &ms)) {
+                }, 0, 0, &ms)) {
                 (void)cudaGetLastError();
                 return CUDEC_ERR_CUDA;
             }
@@ -634,16 +674,29 @@ cudec_status cudec_mixed_plan_tune(cudec_mixed_plan* plan, const void* const* d_
             timed([&] {
                 cdb::mixed::mixed_kernel<<<plan->grid, cdb::mixed::kThreads, cdb::mixed::kSmem,
                                            plan->s>>>(a);
-            }, 0, &warp_ms) &&
+            }, 0, 0, &warp_ms) &&
             timed([&] {
                 cdb::mixed::mixed_cta_kernel<<<cg, cdb::lzc::kThreads, cdb::mixed::kCtaSmem,
                                                plan->s>>>(make_cta_args(plan, whole));
-            }, l.size(), &cta_ms);
+            }, 0, l.size(), &cta_ms);
         if (!ok) {
             (void)cudaGetLastError();
             return CUDEC_ERR_CUDA;
         }
         plan->wpc[bk] = cta_ms < warp_ms ? cdb::mixed::kCtaWarps : 1u;
+    }
+    if (!zs.empty()) {  // destinations and results receive the whole batch's decode
+        float ms = 0.f;
+        const unsigned zg = static_cast<unsigned>(std::min<size_t>(zs.size(), plan->zstd_grid));
+        if (cudaMemcpyAsync(plan->order.p, zs.data(), zs.size() * sizeof(uint32_t),
+                            cudaMemcpyHostToDevice, plan->s) != cudaSuccess ||
+            !timed([&] {
+                cdb::mixed::mixed_zstd_kernel<<<zg, cdb::zstd::kTeam, 0, plan->s>>>(
+                    make_cta_args(plan, whole));
+            }, zs.size(), zs.size(), &ms)) {
+            (void)cudaGetLastError();
+            return CUDEC_ERR_CUDA;
+        }
     }
     return cudaStreamSynchronize(plan->s) == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
 }

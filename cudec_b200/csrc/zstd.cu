@@ -15,33 +15,30 @@ namespace cdb {
 namespace zstd {
 
 constexpr uint32_t kMaxSlots = 4096;  // frames decoded concurrently (workspace slots)
+constexpr uint32_t kSlotGroup = 4;    // the workspace holds a multiple of these
+// Resident CTAs per SM that the registers are compiled for: with 3 a lone frame
+// is quicker (six frames of 128 KiB 825 us against 877) but 512 frames of
+// 1 MiB take 10,716 us against 7,846; 5 cost registers and were slower on
+// both.
+constexpr uint32_t kTeamsPerSm = 4;
 
-// Multi: a chunk is a sequence of frames (decode_frames) rather than one
-// frame (decode_frame); a template parameter, so the one-frame kernel is
-// compiled alone.
+// One CTA per frame in flight. Multi: a chunk is a sequence of frames
+// (decode_frames) rather than one frame (decode_frame); a template parameter,
+// so the one-frame kernel is compiled alone.
 template <bool Multi>
-__global__ void __launch_bounds__(kCtaThreads)
+__global__ void __launch_bounds__(kTeam, kTeamsPerSm)
     zstd_decode_kernel(const void* const* src_ptrs, const size_t* src_sizes,
                        void* const* dst_ptrs, const size_t* dst_caps, size_t n,
                        cudec_chunk_result* results, uint8_t* workspace) {
-    __shared__ WarpSmem wsm[kWarpsPerCta];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const size_t gw = static_cast<size_t>(blockIdx.x) * kWarpsPerCta + warp;
-    const size_t total = static_cast<size_t>(gridDim.x) * kWarpsPerCta;
-    uint8_t* litbuf = workspace + gw * kLitSlot;
-    for (size_t c = gw; c < n; c += total) {
+    __shared__ TeamSmem s;
+    uint8_t* slot = workspace + static_cast<size_t>(blockIdx.x) * kLitSlot;
+    for (size_t c = blockIdx.x; c < n; c += gridDim.x) {
         uint64_t written = 0;
         const uint8_t* src = static_cast<const uint8_t*>(src_ptrs[c]);
         uint8_t* dst = static_cast<uint8_t*>(dst_ptrs[c]);
-        int st;
-        if constexpr (Multi)
-            st = decode_frames(src, src_sizes[c], dst, dst_caps[c], wsm[warp], litbuf, lane,
-                               &written);
-        else
-            st = decode_frame(src, src_sizes[c], dst, dst_caps[c], wsm[warp], litbuf, lane,
-                              &written);
-        __syncwarp();
-        if (lane == 0) {
+        const int st = Multi ? decode_frames(src, src_sizes[c], dst, dst_caps[c], s, slot, &written)
+                             : decode_frame(src, src_sizes[c], dst, dst_caps[c], s, slot, &written);
+        if (threadIdx.x == 0) {
             results[c].status = st;
             results[c].reserved = 0;
             results[c].bytes_written = st == CUDEC_OK ? written : 0;
@@ -56,8 +53,8 @@ extern "C" {
 
 size_t cudec_zstd_workspace_bytes(size_t chunk_count) {
     const size_t slots = chunk_count < cdb::zstd::kMaxSlots ? chunk_count : cdb::zstd::kMaxSlots;
-    const size_t rounded = (slots + cdb::zstd::kWarpsPerCta - 1) / cdb::zstd::kWarpsPerCta *
-                           cdb::zstd::kWarpsPerCta;
+    const size_t rounded = (slots + cdb::zstd::kSlotGroup - 1) / cdb::zstd::kSlotGroup *
+                           cdb::zstd::kSlotGroup;
     return rounded * cdb::zstd::kLitSlot;
 }
 
@@ -75,11 +72,11 @@ cudec_status launch_zstd(const void* const* d_src_ptrs, const size_t* d_src_size
     if (d_workspace == nullptr || workspace_bytes < cudec_zstd_workspace_bytes(chunk_count))
         return CUDEC_ERR_INVALID_ARGUMENT;
     (void)cudaGetLastError();
-    const size_t slots = cudec_zstd_workspace_bytes(chunk_count) / cdb::zstd::kLitSlot;
-    const unsigned grid = static_cast<unsigned>(slots / cdb::zstd::kWarpsPerCta);
+    const unsigned grid = static_cast<unsigned>(
+        chunk_count < cdb::zstd::kMaxSlots ? chunk_count : cdb::zstd::kMaxSlots);
     const auto kernel = multi ? cdb::zstd::zstd_decode_kernel<true>
                               : cdb::zstd::zstd_decode_kernel<false>;
-    kernel<<<grid, cdb::zstd::kCtaThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+    kernel<<<grid, cdb::zstd::kTeam, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         d_src_ptrs, d_src_sizes, d_dst_ptrs, d_dst_capacities, chunk_count, d_results,
         static_cast<uint8_t*>(d_workspace));
     return cudaGetLastError() == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
@@ -128,7 +125,6 @@ namespace zstd {
 
 constexpr size_t kNoAllocChunks = CUDEC_ZSTD_NOALLOC_MAX_CHUNKS;
 constexpr int kNoAllocMaxDevices = 256;
-static_assert(kNoAllocChunks % kWarpsPerCta == 0, "whole CTAs of slots");
 
 static __device__ __align__(256) uint8_t g_noalloc_slots[kNoAllocChunks * kLitSlot];
 
@@ -173,10 +169,8 @@ extern "C" cudec_status cudec_zstd_decompress_batch_noalloc(
         (void)cudaGetLastError();
         return CUDEC_ERR_CUDA;
     }
-    const unsigned grid = static_cast<unsigned>(
-        (chunk_count + cdb::zstd::kWarpsPerCta - 1) / cdb::zstd::kWarpsPerCta);
-    cdb::zstd::zstd_decode_kernel<false><<<grid, cdb::zstd::kCtaThreads, 0,
-                                           reinterpret_cast<cudaStream_t>(stream)>>>(
+    cdb::zstd::zstd_decode_kernel<false><<<static_cast<unsigned>(chunk_count), cdb::zstd::kTeam,
+                                           0, reinterpret_cast<cudaStream_t>(stream)>>>(
         d_src_ptrs, d_src_sizes, d_dst_ptrs, d_dst_capacities, chunk_count, d_results, slots);
     return cudaGetLastError() == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
 }

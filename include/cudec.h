@@ -240,8 +240,8 @@ typedef enum cudec_format {
  * < 16 KiB, < 64 KiB, < 256 KiB, < 1 MiB, larger. */
 #define CUDEC_MIXED_BUCKETS 6
 
-/* Warps of the CTA-per-chunk LZ4 / Snappy decoder (the whole-CTA value of a
- * decode shape's warps per chunk). */
+/* The value of a decode shape's warps per chunk that names the CTA-per-chunk
+ * LZ4 / Snappy decoder (which picks its own width). */
 #define CUDEC_MIXED_CTA_WARPS 8
 
 typedef struct cudec_mixed_plan cudec_mixed_plan;

@@ -277,7 +277,8 @@ inline uint32_t lds(SAddr a) {
     in_smem(a, 4);
     return *reinterpret_cast<const uint32_t*>(a);
 }
-inline void sts4(SAddr a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+inline void sts4_first(SAddr a, uint32_t x, uint32_t y, uint32_t z, uint32_t w, uint32_t lane) {
+    if (lane) return;
     in_smem(a, 16);
     uint32_t* p = reinterpret_cast<uint32_t*>(a);
     p[0] = x, p[1] = y, p[2] = z, p[3] = w;

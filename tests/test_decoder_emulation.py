@@ -5,9 +5,11 @@ collectives and barriers (a deadlock, lanes at different collectives, or
 threads that disagree on the result fail the run), in an order drawn from a
 seed. The sizes are those where the decoders change their way: LZ4 and Snappy
 chunks of one tile and of several at each width of the CTA, batches cut by
-long tokens, tiles that few tokens settle; short GDeflate pages and full ones.
-Statuses, bytes and untouched memory around them equal the oracle's; the
-mutants cover the early ends.
+long tokens, tiles that few tokens settle; Zstd frames of no, one and more
+than one item of 128 sequences, one and several blocks, literal streams shared
+by eight lanes or not, runs longer than a lane's own copies; short GDeflate
+pages and full ones. Statuses, bytes and untouched memory around them equal
+the oracle's; the mutants cover the early ends.
 """
 import ctypes
 import os
@@ -50,6 +52,22 @@ def lz():
         return lambda src, n, dst, cap, seed, written: lib.lz_emulate(
             fmt, threads, src, n, dst, cap, seed, written)
     return call
+
+
+@pytest.fixture(scope="module")
+def zstd():
+    lib = _build("zstd_emul")
+    lib.zstd_emulate.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p,
+                                 ctypes.c_uint64, ctypes.c_void_p, ctypes.c_uint64,
+                                 ctypes.POINTER(ctypes.c_uint64)]
+    slot = np.zeros(128 * 1024, dtype=np.uint8)
+
+    def call(multi):
+        def run(src, n, dst, cap, seed, written):
+            slot[:] = 0xEE
+            return lib.zstd_emulate(multi, src, n, dst, cap, slot.ctypes.data, seed, written)
+        return run
+    return {"one": call(0), "multi": call(1)}
 
 
 @pytest.fixture(scope="module")
@@ -124,6 +142,31 @@ def test_lz(lz, size, threads):
             for m in range(4 if size < 6000 else 1):
                 check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2, m, 0,
                       (size, k, fmt, m))
+
+
+@pytest.mark.parametrize("size", [0, 1, 40, 1000, 1600, 9000, 131072, 150000])
+def test_zstd(zstd, size):
+    for k, data in enumerate(contents(size)):
+        for level in (1, 19):
+            f = W.zstd_compress(data, level, 20, level == 19)
+            check(zstd["one"], oracle.zstd_decode, f, size, k, (5 * k + level) % 16,
+                  (size, k, level))
+    check(zstd["one"], oracle.zstd_decode, f, size + 9, 3, 1, (size, "room"))
+
+
+def test_zstd_mutants(zstd):
+    rng = random.Random(11)
+    frames = [(W.zstd_compress(d, lv, 20, True), size) for size in (300, 4000, 140000)
+              for lv in (1, 19) for d in contents(size)]
+    for k in range(240):
+        f, cap = frames[k % len(frames)]
+        if cap > 100000 and k % 3:
+            continue
+        cut = rng.choice([0, 0, 1, cap // 2])
+        check(zstd["one"], oracle.zstd_decode, mutate(rng, f), cap - cut, k, k % 16, k)
+        if k % 5 == 0:
+            two = f + b"\x50\x2a\x4d\x18\x03\x00\x00\x00abc" + mutate(rng, frames[0][0])
+            check(zstd["multi"], oracle.zstd_decode_multi, two, 2 * cap, k, 0, ("multi", k))
 
 
 @pytest.mark.parametrize("size", [0, 1, 63, 3000, 20000, 65536])
