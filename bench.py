@@ -929,7 +929,7 @@ def main():
             **({"reference_gpu": ref_gpu} if ref_gpu else {}),
             **({"mixed": mixed_line} if mixed_line else {}),
             **({"serve": serve_line} if serve_line else {}),
-            "gpu_launches": args.steps,
+            "gpu_launches": 2 * args.steps,  # wide and narrow CTAs (more than 3 chunks per SM)
             "clocks": clocks.summary(),
         }
         if world == 1 and args.cpu_seconds > 0:

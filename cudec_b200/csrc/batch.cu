@@ -40,6 +40,10 @@ std::atomic<int> g_sm_count[kMaxDevices];
 // 337, 592 chunks 527 / 393 / 357, 1,024 chunks 856 / 563 / 447; 16 chunks of
 // 4 MiB 9,550 / 11,720 / 15,980.
 constexpr size_t kWideMax = 1, kMediumMax = 3;
+constexpr uint32_t kWideThreads = 256;  // beside narrow CTAs
+// Up to here a wide CTA reads every capacity (148 x 1 MiB out of L2, some 30 us
+// of a launch that takes many milliseconds).
+constexpr size_t kWideBeside = 1 << 17;
 
 }  // namespace
 
@@ -53,16 +57,20 @@ int device_sm_count(int dev) {
     return v;
 }
 
-// The kernel's shared state exceeds 48 KB: opted into once per device, format
+// The kernels' shared state exceeds 48 KB: opted into once per device, format
 // and width.
 template <class F, uint32_t T>
 cudaError_t prepare_cta(int dev) {
     static std::atomic<bool> ready[kMaxDevices];
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     if (ready[dev].load(std::memory_order_acquire)) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(lzc::lz_cta_kernel<F, T>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(sizeof(lzc::Shm<F, T>)));
+    constexpr int kSmem = static_cast<int>(sizeof(lzc::Shm<F, T>));
+    cudaError_t e = cudaFuncSetAttribute(lzc::lz_cta_kernel<F, T>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if constexpr (T == kWideThreads)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(lzc::lz_wide_kernel<F, T>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     if (e == cudaSuccess) ready[dev].store(true, std::memory_order_release);
     return e;
 }
@@ -86,8 +94,37 @@ cudec_status launch_width(const Batch& b) {
     constexpr size_t kMaxGrid = INT32_MAX;
     const unsigned grid = static_cast<unsigned>(b.n < kMaxGrid ? b.n : kMaxGrid);
     lzc::lz_cta_kernel<F, T><<<grid, T, sizeof(lzc::Shm<F, T>), b.stream>>>(
-        b.src, b.src_sizes, b.dst, b.caps, b.n, b.results);
+        b.src, b.src_sizes, b.dst, b.caps, b.n, b.results, 0);
     return cudaGetLastError() == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
+}
+
+// Many chunks: narrow CTAs, and beside them a wide CTA per SM for the few
+// that are large (lz_wide_kernel). The narrow kernel is a programmatic
+// dependent of the wide one, which lets it start at once.
+template <class F>
+cudec_status launch_many(const Batch& b, unsigned sms) {
+    if (prepare_cta<F, 128>(b.dev) != cudaSuccess ||
+        prepare_cta<F, kWideThreads>(b.dev) != cudaSuccess)
+        return CUDEC_ERR_CUDA;
+    lzc::lz_wide_kernel<F, kWideThreads>
+        <<<sms, kWideThreads, sizeof(lzc::Shm<F, kWideThreads>), b.stream>>>(
+            b.src, b.src_sizes, b.dst, b.caps, b.n, b.results);
+    if (cudaGetLastError() != cudaSuccess) return CUDEC_ERR_CUDA;
+    constexpr size_t kMaxGrid = INT32_MAX;
+    cudaLaunchAttribute beside{};
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(b.n < kMaxGrid ? b.n : kMaxGrid));
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = sizeof(lzc::Shm<F, 128>);
+    cfg.stream = b.stream;
+    cfg.attrs = &beside;
+    cfg.numAttrs = 1;
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, lzc::lz_cta_kernel<F, 128>, b.src, b.src_sizes, b.dst, b.caps,
+                           b.n, b.results, static_cast<uint32_t>(sms));
+    return e == cudaSuccess ? CUDEC_OK : CUDEC_ERR_CUDA;
 }
 
 template <class F>
@@ -105,6 +142,7 @@ cudec_status launch_lz_cta(const void* const* src, const size_t* src_sizes, void
     // wide while the batch leaves SMs idle otherwise.
     if (n <= kWideMax * sms) return launch_width<F, 512>(b);
     if (n <= kMediumMax * sms) return launch_width<F, 256>(b);
+    if (n <= kWideBeside) return launch_many<F>(b, static_cast<unsigned>(sms));
     return launch_width<F, 128>(b);
 }
 

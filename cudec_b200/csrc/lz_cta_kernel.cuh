@@ -1029,26 +1029,122 @@ struct Chunk {
 };
 
 // ---------------------------------------------------------------------------
-// The batch kernel: one CTA per chunk. Dynamic shared memory: sizeof(Shm).
+// The batch kernels. Dynamic shared memory: sizeof(Shm).
 #if defined(__CUDACC__)
+// In a batch of many chunks a few large ones would run on alone at the
+// narrow CTAs' pace: those are left to a CTA each of the wide kernel that runs
+// beside. Large: a capacity of 2^k bytes or more, for the smallest k from
+// kLargeLog on that leaves no more of them than the wide kernel has CTAs (a
+// batch of many large chunks has the SMs busy to its end anyway). Measured:
+// 8,000 uneven Snappy chunks (256 bytes to 4 MiB, median 16 KiB) 7,997 us
+// without the wide kernel, 4,950 with it; 2,000 of them 4,084 and 2,610;
+// 30,000 uneven LZ4 chunks 5,901 and 3,811, with kLargeLog 19 4,022, with 17
+// the same. Where no chunk is large the count of them costs 2 us in 410
+// (1,024 chunks) to 8 in 443 (8,192).
+constexpr uint32_t kLargeLog = 18, kLogs = 16;
+
+// The k - kLargeLog of the batch (kLogs: no chunk is large), by the whole CTA;
+// count: the large chunks.
+__device__ __forceinline__ uint32_t large_from(const size_t* caps, size_t n, uint32_t wide,
+                                               uint32_t* count) {
+    __shared__ uint32_t hist[kLogs];
+    if (threadIdx.x < kLogs) hist[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll 8
+    for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint64_t c = caps[i];
+        if (c >> kLargeLog) {
+            const uint32_t k = 63 - kLargeLog - __clzll(static_cast<long long>(c));
+            atomicAdd(&hist[k < kLogs ? k : kLogs - 1], 1u);
+        }
+    }
+    __syncthreads();
+    uint32_t k = kLogs, sum = 0;
+    while (k != 0 && hist[k - 1] <= wide - sum) sum += hist[--k];
+    __syncthreads();  // read by every thread before the next use
+    *count = sum;
+    return sum ? k : kLogs;
+}
+__device__ __forceinline__ bool is_large(uint64_t cap, uint32_t k) {
+    return k < kLogs && (cap >> (kLargeLog + k)) != 0;
+}
+
+// The index of the batch's large chunk number w (threads' shares in turn), by
+// the whole CTA of T threads; w < their count.
+template <uint32_t T>
+__device__ __forceinline__ size_t large_chunk(const size_t* caps, size_t n, uint32_t k,
+                                              uint32_t w) {
+    __shared__ uint32_t sums[T / 32];
+    __shared__ size_t found;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint32_t mine = 0;
+#pragma unroll 4
+    for (size_t i = t; i < n; i += T) mine += is_large(caps[i], k);
+    uint32_t before = mine;  // then inclusive over the warp
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, before, d);
+        if (lane >= d) before += v;
+    }
+    if (lane == 31) sums[warp] = before;
+    __syncthreads();
+    for (uint32_t i = 0; i < warp; ++i) before += sums[i];
+    if (w < before && w >= before - mine) {
+        uint32_t left = w - (before - mine);
+        size_t i = t;
+        while (!is_large(caps[i], k) || left-- != 0) i += T;
+        found = i;
+    }
+    __syncthreads();
+    return found;
+}
+
+template <class F, uint32_t kThreads>
+__device__ __forceinline__ void decode_chunk(size_t c, const void* const* src_ptrs,
+                                             const size_t* src_sizes, void* const* dst_ptrs,
+                                             const size_t* dst_caps, cudec_chunk_result* results) {
+    extern __shared__ __align__(16) uint8_t lzc_smem[];
+    Shm<F, kThreads>& s = *reinterpret_cast<Shm<F, kThreads>*>(lzc_smem);
+    Chunk<F, kThreads> ch{s, static_cast<const uint8_t*>(src_ptrs[c]), src_sizes[c],
+                          static_cast<uint8_t*>(dst_ptrs[c]), dst_caps[c], 0};
+    uint64_t written = 0;
+    const int st = ch.run(&written);
+    if (threadIdx.x == 0) {
+        results[c].status = st;
+        results[c].reserved = 0;
+        results[c].bytes_written = st == CUDEC_OK ? written : 0;
+    }
+    __syncthreads();  // the next chunk reuses the shared state
+}
+
+// One CTA per chunk. wide: the wide kernel's CTAs (0: it does not run).
 template <class F, uint32_t kThreads>
 __global__ void __launch_bounds__(kThreads, Width<kThreads>::kPerSm)
     lz_cta_kernel(const void* const* src_ptrs, const size_t* src_sizes, void* const* dst_ptrs,
-                  const size_t* dst_caps, size_t n, cudec_chunk_result* results) {
-    extern __shared__ __align__(16) uint8_t lzc_smem[];
-    Shm<F, kThreads>& s = *reinterpret_cast<Shm<F, kThreads>*>(lzc_smem);
+                  const size_t* dst_caps, size_t n, cudec_chunk_result* results, uint32_t wide) {
+    uint32_t count;
     for (size_t c = blockIdx.x; c < n; c += gridDim.x) {
-        Chunk<F, kThreads> ch{s, static_cast<const uint8_t*>(src_ptrs[c]), src_sizes[c],
-                              static_cast<uint8_t*>(dst_ptrs[c]), dst_caps[c], 0};
-        uint64_t written = 0;
-        const int st = ch.run(&written);
-        if (threadIdx.x == 0) {
-            results[c].status = st;
-            results[c].reserved = 0;
-            results[c].bytes_written = st == CUDEC_OK ? written : 0;
-        }
-        __syncthreads();  // the next chunk reuses the shared state
+        if (wide && (dst_caps[c] >> kLargeLog) &&
+            is_large(dst_caps[c], large_from(dst_caps, n, wide, &count)))
+            continue;  // a wide CTA's
+        decode_chunk<F, kThreads>(c, src_ptrs, src_sizes, dst_ptrs, dst_caps, results);
     }
+    // the two kernels end together: this one is launched without waiting for
+    // the wide one, which has all its CTAs running or done by now
+    if (wide && blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class F, uint32_t kThreads>
+__global__ void __launch_bounds__(kThreads, Width<kThreads>::kPerSm)
+    lz_wide_kernel(const void* const* src_ptrs, const size_t* src_sizes, void* const* dst_ptrs,
+                   const size_t* dst_caps, size_t n, cudec_chunk_result* results) {
+    uint32_t count;
+    const uint32_t k = large_from(dst_caps, n, gridDim.x, &count);
+    // a CTA without work leaves first, so that the narrow ones spread evenly
+    if (blockIdx.x >= count) return;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    decode_chunk<F, kThreads>(large_chunk<kThreads>(dst_caps, n, k, blockIdx.x), src_ptrs,
+                              src_sizes, dst_ptrs, dst_caps, results);
 }
 #endif
 

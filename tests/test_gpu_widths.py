@@ -61,3 +61,56 @@ def test_widths(cuda, fmt, n):
         if st == 0:
             assert res[i]["bytes_written"] == len(out)
             assert b.output(i, dst) == out + b"\xa5" * (caps[i] - len(out)), i
+
+
+@pytest.mark.parametrize("fmt", ["lz4", "snappy"])
+@pytest.mark.parametrize("large", [1, 147, 148, 149, 500])
+def test_large_among_many(cuda, fmt, large):
+    """Chunks of 256 KiB of capacity and more beside many small ones: up to one
+    per SM go to wide CTAs, past that those of 512 KiB and more, and so on."""
+    import torch
+    n = 500
+    raws = [r[:3000] for r in chunks(n)]
+    rng = random.Random(large)
+    caps = [len(r) for r in raws]
+    for j, i in enumerate(rng.sample(range(n), large)):
+        caps[i] = (262144, 262145, 524287, 524288, 1 << 20)[j % 5]
+        if j < 3:
+            raws[i] = W.generate([caps[i]], W.lz_params(0.5), seeds=[j])[0].tobytes()
+    comps = [PACK[fmt](r) for r in raws]
+    b = bytearray(comps[7])
+    b[len(b) // 2] ^= 4
+    comps[7] = bytes(b)
+    b = DeviceBatch(comps, caps, device=cuda, dst_align=16, dst_skew=3, src_skew=5)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    for _ in range(2):
+        assert b.run(fmt, stream) == 0
+    stream.synchronize()
+    res, dst = b.results(), b.dst_host()
+    for i in range(n):
+        st, out = WANT[fmt](comps[i], caps[i])
+        assert res[i]["status"] == st, (i, res[i], st)
+        if st == 0:
+            assert res[i]["bytes_written"] == len(out)
+            assert b.output(i, dst) == out + b"\xa5" * (caps[i] - len(out)), i
+
+
+def test_large_among_many_captured(cuda):
+    import torch
+    raws = [r[:3000] for r in chunks(450)]
+    raws[33] = W.generate([300000], W.lz_params(0.5), seeds=[1])[0].tobytes()
+    b = DeviceBatch([PACK["lz4"](r) for r in raws], [len(r) for r in raws], device=cuda)
+    assert b.run("lz4") == 0
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert b.run("lz4") == 0
+    b.d_dst.zero_()
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    dst = b.dst_host()
+    assert (b.results()["status"] == 0).all()
+    for i, r in enumerate(raws):
+        assert b.output(i, dst) == r, i
