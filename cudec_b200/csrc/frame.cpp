@@ -18,8 +18,10 @@
 
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <new>
 #include <thread>
 #include <vector>
@@ -114,6 +116,73 @@ class BlockSums {
     bool ok_ = true;
 };
 
+// The content checksum beside the copy back: a thread hashes the output as it
+// arrives in order. begin() starts it (without a thread to be had the calling
+// thread hashes in finish()); grown() says how much is in place.
+class ContentSum {
+  public:
+    ContentSum() = default;
+    ~ContentSum() { stop(); }
+    ContentSum(const ContentSum&) = delete;
+    ContentSum& operator=(const ContentSum&) = delete;
+
+    void begin(const unsigned char* out) {
+        out_ = out;
+        try {
+            thread_ = std::thread([this] { run(); });
+        } catch (...) {
+        }
+    }
+    void grown(size_t n) {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            ready_ = n;
+        }
+        cv_.notify_one();
+    }
+    uint32_t finish(const unsigned char* out, size_t total) {
+        if (thread_.joinable()) grown(total);
+        stop();
+        sum_.stripes(out + done_, (total - done_) / 16);
+        return sum_.finish(out + total / 16 * 16, total % 16);
+    }
+
+  private:
+    void run() {
+        std::unique_lock<std::mutex> lk(mu_);
+        for (;;) {
+            cv_.wait(lk, [this] { return ended_ || ready_ - done_ >= 16; });
+            const size_t n = (ready_ - done_) / 16;
+            if (n == 0) return;
+            lk.unlock();
+            sum_.stripes(out_ + done_, n);
+            done_ += 16 * n;
+            lk.lock();
+        }
+    }
+    void stop() {
+        if (!thread_.joinable()) return;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            ended_ = true;
+        }
+        cv_.notify_one();
+        thread_.join();
+    }
+
+    const unsigned char* out_ = nullptr;
+    std::thread thread_;
+    std::mutex mu_;
+    std::condition_variable cv_;
+    size_t ready_ = 0;  // under mu_
+    bool ended_ = false;
+    size_t done_ = 0;   // the thread's, then (joined) the caller's
+    cdb::Xxh32 sum_;
+};
+
+// The copy back goes in parts of this size when a checksum follows it.
+constexpr size_t kCopyPart = size_t{4} << 20;
+
 #define FCUDA(call)                                   \
     do {                                              \
         if ((call) != cudaSuccess) {                  \
@@ -132,7 +201,8 @@ class BlockSums {
 // when the walk itself rejects the block.
 cudec_status decode_blocks(const unsigned char* f, const std::vector<Block>& blocks,
                            size_t block_max, unsigned char* out, size_t cap,
-                           size_t* total_out, const std::function<bool()>& sums_ok) {
+                           size_t* total_out, const std::function<bool()>& sums_ok,
+                           ContentSum* content) {
     std::vector<size_t> comp;
     for (size_t i = 0; i < blocks.size(); ++i)
         if (!blocks[i].raw) comp.push_back(i);
@@ -191,21 +261,44 @@ cudec_status decode_blocks(const unsigned char* f, const std::vector<Block>& blo
         if (len > cap - total) return CUDEC_ERR_OUTPUT_TOO_SMALL;
         total += len;
     }
-    // Place blocks; merge device runs that are contiguous on both sides.
+    // Place blocks; merge device runs that are contiguous on both sides. With
+    // a content checksum to follow, runs go in parts, each in place before
+    // the next, and the checksum runs behind them.
+    if (content != nullptr && total >= 2 * kCopyPart) content->begin(out);
+    else content = nullptr;
     size_t run_dev = 0, run_out = 0, run_len = 0, off = 0, k = 0;
+    const auto copy_run = [&]() -> cudec_status {
+        for (size_t at = 0; at < run_len;) {
+            const size_t len = content ? std::min(kCopyPart, run_len - at) : run_len;
+            FCUDA(cudaMemcpyAsync(out + run_out + at,
+                                  static_cast<unsigned char*>(d_dst.p) + run_dev + at, len,
+                                  cudaMemcpyDeviceToHost, stream.s));
+            at += len;
+            if (content) {
+                FCUDA(cudaStreamSynchronize(stream.s));
+                content->grown(run_out + at);
+            }
+        }
+        run_len = 0;
+        return CUDEC_OK;
+    };
     for (size_t i = 0; i < blocks.size(); ++i) {
         if (blocks[i].raw) {
+            if (content) {  // in order
+                const cudec_status st = copy_run();
+                if (st != CUDEC_OK) return st;
+            }
             if (blocks[i].len) std::memcpy(out + off, f + blocks[i].off, blocks[i].len);
             off += blocks[i].len;
+            if (content) content->grown(off);
             continue;
         }
         const size_t len = dec_len[i], dev = k * block_max;
         if (run_len != 0 && run_dev + run_len == dev && run_out + run_len == off) {
             run_len += len;
         } else {
-            if (run_len)
-                FCUDA(cudaMemcpyAsync(out + run_out, static_cast<unsigned char*>(d_dst.p) + run_dev,
-                                      run_len, cudaMemcpyDeviceToHost, stream.s));
+            const cudec_status st = copy_run();
+            if (st != CUDEC_OK) return st;
             run_dev = dev;
             run_out = off;
             run_len = len;
@@ -213,9 +306,8 @@ cudec_status decode_blocks(const unsigned char* f, const std::vector<Block>& blo
         off += len;
         ++k;
     }
-    if (run_len)
-        FCUDA(cudaMemcpyAsync(out + run_out, static_cast<unsigned char*>(d_dst.p) + run_dev,
-                              run_len, cudaMemcpyDeviceToHost, stream.s));
+    const cudec_status placed = copy_run();
+    if (placed != CUDEC_OK) return placed;
     if (n) FCUDA(cudaStreamSynchronize(stream.s));
     *total_out = total;
     return CUDEC_OK;
@@ -271,15 +363,17 @@ cudec_status decode_frame(const unsigned char* f, size_t size, unsigned char* ou
     size_t total = 0;
     // the checksum values are verified while the blocks decode
     BlockSums sums(f, blocks, block_sum);
-    const cudec_status st =
-        decode_blocks(f, blocks, block_max, out, cap, &total, [&sums] { return sums.ok(); });
+    ContentSum content;
+    const cudec_status st = decode_blocks(f, blocks, block_max, out, cap, &total,
+                                          [&sums] { return sums.ok(); },
+                                          content_sum ? &content : nullptr);
     // a checksum mismatch outranks whatever the device path met (the walk
     // would have stopped before any CUDA call)
     if (st != CUDEC_OK) return sums.ok() ? st : CUDEC_ERR_CORRUPT_INPUT;
     if (has_size && declared != total) return CUDEC_ERR_CORRUPT_INPUT;
     if (content_sum) {
         if (size < pos + 4) return CUDEC_ERR_CORRUPT_INPUT;
-        if (xxh32(out, total) != rd32(f + pos)) return CUDEC_ERR_CORRUPT_INPUT;
+        if (content.finish(out, total) != rd32(f + pos)) return CUDEC_ERR_CORRUPT_INPUT;
     }
     *written = total;
     return CUDEC_OK;

@@ -26,40 +26,52 @@ inline uint32_t xxh_read32(const unsigned char* p) {
     return v;
 }
 
-inline uint32_t xxh32(const void* data, size_t len, uint32_t seed = 0) {
-    const unsigned char* p = static_cast<const unsigned char*>(data);
-    const unsigned char* const end = p + len;
-    uint32_t h;
-    if (len >= 16) {
-        uint32_t a = seed + kXxhP1 + kXxhP2, b = seed + kXxhP2, c = seed,
-                 d = seed - kXxhP1;
-        const unsigned char* const limit = end - 16;
-        do {
+// The digest of data that arrives in parts: stripes() takes whole 16-byte
+// stripes, finish() the rest.
+class Xxh32 {
+  public:
+    explicit Xxh32(uint32_t seed = 0)
+        : seed_(seed), v_{seed + kXxhP1 + kXxhP2, seed + kXxhP2, seed, seed - kXxhP1} {}
+
+    void stripes(const unsigned char* p, size_t n) {  // n stripes
+        len_ += 16 * static_cast<uint64_t>(n);
+        uint32_t a = v_[0], b = v_[1], c = v_[2], d = v_[3];
+        for (; n != 0; --n, p += 16) {
             a = xxh_rotl(a + xxh_read32(p) * kXxhP2, 13) * kXxhP1;
             b = xxh_rotl(b + xxh_read32(p + 4) * kXxhP2, 13) * kXxhP1;
             c = xxh_rotl(c + xxh_read32(p + 8) * kXxhP2, 13) * kXxhP1;
             d = xxh_rotl(d + xxh_read32(p + 12) * kXxhP2, 13) * kXxhP1;
-            p += 16;
-        } while (p <= limit);
-        h = xxh_rotl(a, 1) + xxh_rotl(b, 7) + xxh_rotl(c, 12) + xxh_rotl(d, 18);
-    } else {
-        h = seed + kXxhP5;
+        }
+        v_[0] = a, v_[1] = b, v_[2] = c, v_[3] = d;
     }
-    h += static_cast<uint32_t>(len);
-    while (p + 4 <= end) {
-        h = xxh_rotl(h + xxh_read32(p) * kXxhP3, 17) * kXxhP4;
-        p += 4;
+
+    uint32_t finish(const unsigned char* p, size_t rest) {  // rest < 16
+        uint32_t h = len_ != 0 ? xxh_rotl(v_[0], 1) + xxh_rotl(v_[1], 7) + xxh_rotl(v_[2], 12) +
+                                     xxh_rotl(v_[3], 18)
+                               : seed_ + kXxhP5;
+        h += static_cast<uint32_t>(len_ + rest);
+        const unsigned char* const end = p + rest;
+        for (; p + 4 <= end; p += 4) h = xxh_rotl(h + xxh_read32(p) * kXxhP3, 17) * kXxhP4;
+        for (; p < end; ++p) h = xxh_rotl(h + (*p) * kXxhP5, 11) * kXxhP1;
+        h ^= h >> 15;
+        h *= kXxhP2;
+        h ^= h >> 13;
+        h *= kXxhP3;
+        h ^= h >> 16;
+        return h;
     }
-    while (p < end) {
-        h = xxh_rotl(h + (*p) * kXxhP5, 11) * kXxhP1;
-        ++p;
-    }
-    h ^= h >> 15;
-    h *= kXxhP2;
-    h ^= h >> 13;
-    h *= kXxhP3;
-    h ^= h >> 16;
-    return h;
+
+  private:
+    uint32_t seed_;
+    uint32_t v_[4];
+    uint64_t len_ = 0;
+};
+
+inline uint32_t xxh32(const void* data, size_t len, uint32_t seed = 0) {
+    const unsigned char* p = static_cast<const unsigned char*>(data);
+    Xxh32 h(seed);
+    h.stripes(p, len / 16);
+    return h.finish(p + len / 16 * 16, len % 16);
 }
 
 }  // namespace cdb
