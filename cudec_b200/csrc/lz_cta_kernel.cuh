@@ -14,18 +14,24 @@
 //      from every position of a region (kReg positions, one region per
 //      thread) the distance to the first chain position past the region,
 //      computed backwards;
-//   3. settle: region t is entered at region t - 1's exit. Every region
-//      starts from the exit of its first position; LZ chains started
-//      anywhere merge after a few tokens, so most are right at once. In a
-//      round, the first region f whose entry is not its neighbour's exit
-//      takes it (everything before f is right), a region that the chain
-//      leaving f - 1 passes over takes that exit too, and any other region
-//      takes its neighbour's exit where that lies inside it; each looks its
-//      own exit up. Only region f takes an uncommon step (a long extension,
-//      the chunk's end), the others leave it open, to be taken when they are
-//      first. Rounds repeat until every region is settled; after kRounds of
-//      them (content with few tokens per region) one thread follows the
-//      chain through the rest, a look-up per region;
+//   3. the regions' entries: region t is entered at region t - 1's exit. LZ
+//      chains started anywhere merge after a few tokens, which two ways use:
+//      settle (CTAs up to kSettle threads): every region starts from the exit
+//      of its first position, so most are right at once. In a round, the
+//      first region f whose entry is not its neighbour's exit takes it
+//      (everything before f is right), a region that the chain leaving f - 1
+//      passes over takes that exit too, and any other region takes its
+//      neighbour's exit where that lies inside it; each looks its own exit
+//      up. Only region f takes an uncommon step (a long extension, the
+//      chunk's end). After kRounds rounds one thread follows the chain
+//      through the rest, a look-up per region;
+//      chase (wider ones, whose rounds are more and dearer): a warp's 32
+//      regions are followed from each of their first 32 positions at once, one
+//      lane each; lane 0 notes where it enters each region. One thread then
+//      follows the tile's chain from warp to warp: the warp's entry is mostly
+//      one of those 32 positions (or past the warp); otherwise it goes region
+//      by region until it meets the chain of lane 0. Each thread then finds
+//      its region's entry the same way, from its warp's;
 //   4. list: each thread walks its region from its entry; a scan of the
 //      counts gives every token its index, and the tokens' positions go to a
 //      list;
@@ -52,7 +58,7 @@
 // of them in the copy). The decoder before this one computed chain exits by
 // the format's branching step, merged 16-byte pieces per token into a
 // shared-memory ring with atomics, and spent 568,000. 1,024 chunks of 64 KiB
-// on a B200: LZ4 0.943 -> 0.437 ms (154 GB/s out), Snappy 1.149 -> 0.457.
+// on a B200: LZ4 0.943 -> 0.401 ms (167 GB/s out), Snappy 1.149 -> 0.430.
 //
 // Every phase is per-thread code between CTA barriers, driven through an
 // executor: on the device each phase runs once per thread followed by
@@ -110,6 +116,12 @@ constexpr uint32_t kExitMax = 0x80000000u;   // positions are below this
 constexpr uint64_t kStepEnd = ~0ull;
 constexpr uint32_t kSlowRel = 0xFFFFFFFFu;  // a fast step declines: the generic step decides
 constexpr uint32_t kStepSlow = 255;         // no short step from this position
+// Widest CTA whose regions are settled in rounds rather than chased. Us with
+// rounds / chased: 512 threads, 148 LZ4 chunks of 64 KiB 168 / 136, 16 of 4 MiB
+// 9,151 / 6,050 (few tokens per region: 13 rounds and a serial rest per tile);
+// 128 threads, 1,024 Snappy chunks of 64 KiB 430 / 438, 8,192 LZ4 chunks of
+// 8 KiB 453 / 471.
+constexpr uint32_t kSettle = 128;
 constexpr uint32_t kRounds = 12;            // settling rounds before the serial finish
 
 // ---------------------------------------------------------------------------
@@ -131,8 +143,9 @@ inline uint32_t ctz64(uint64_t v) { return static_cast<uint32_t>(__builtin_ctzll
 
 // Profiling builds (-DCDB_PHASE_TIMING) accumulate, from thread 0 of every
 // CTA, the SM cycles of each phase and event counts over a launch. Cycles:
-// 0 stage, 1 steps, 2 exits and settle, 3 list, 4 parse and scan, 5 check and map,
+// 0 stage, 1 steps, 2 exits and entries, 3 list, 4 parse and scan, 5 check and map,
 // 6 copy, 7 whole-CTA tokens. Events: 0 tiles, 1 tokens, 2 settle rounds,
+// regions chased,
 // 3 batches, 4 whole-CTA tokens, 5 windows.
 #if defined(CDB_PHASE_TIMING) && defined(__CUDACC__)
 __device__ unsigned long long lzc_cycles[16];
@@ -505,10 +518,14 @@ struct Shm : Width<kThreads> {
         } e;
         uint8_t period[16 * kThreads];  // whole-CTA copies: a short match's period
     } u;
-    uint32_t exit[kThreads];    // region exits
-    uint32_t entry[kThreads];   // region entries (finish), and which regions are entered
-    uint32_t entered[kWarps];
-    uint32_t votes[kWarps];     // settle: threads whose region is not settled
+    // settle: where each region is left and (finish) entered, which of them
+    // are, and the threads whose region is not settled; chase: where the chain
+    // from a warp's position number `lane` leaves the warp's regions, where
+    // lane 0's enters each of them, where the tile's chain enters the warp's
+    // and leaves the tile
+    uint32_t exit[kThreads], entry[kThreads];
+    uint32_t entered[kWarps], votes[kWarps];
+    uint32_t tile_exit;
     int32_t event[kThreads];    // an event token's ladder status (OK: terminal)
     uint32_t wsum[2][kWarps];   // scans: per-warp totals, used in turn
     Cut cut[2];                 // batches in turn
@@ -687,14 +704,20 @@ struct Chunk {
         return kExitFar;
     }
 
-    // Where the chain through p leaves region t. Not `sure`: p may not be on
-    // the chain, so a way with an uncommon step is left open.
-    CDB_HD uint32_t leave(uint32_t lim, uint32_t rest, uint32_t t, uint32_t p, bool sure) const {
+    // Where the tile's chain, which is at p in region r, leaves the region.
+    CDB_HD uint32_t leave(uint32_t lim, uint32_t rest, uint32_t r, uint32_t p) const {
         const uint32_t d = reinterpret_cast<const uint8_t*>(s.u.w.exit)[p];
         if (d != kStepSlow) return p + d;
-        if (!sure) return kExitOpen;
-        while (p < (t + 1) * kReg) p = hop(lim, rest, p);
+        while (p < (r + 1) * kReg) p = hop(lim, rest, p);
         return p;
+    }
+
+    // Not `sure`: p may not be on the chain, so a way with an uncommon step is
+    // left open.
+    CDB_HD uint32_t leave_if_sure(uint32_t lim, uint32_t rest, uint32_t r, uint32_t p,
+                                  bool sure) const {
+        const uint32_t d = reinterpret_cast<const uint8_t*>(s.u.w.exit)[p];
+        return d != kStepSlow ? p + d : sure ? leave(lim, rest, r, p) : kExitOpen;
     }
 
     // The chain from region f on, entered at `sure`: one thread follows it
@@ -711,28 +734,21 @@ struct Chunk {
                 const uint32_t r = p / kReg;
                 s.entry[r] = p;
                 s.entered[r / 32] |= 1u << (r % 32);
-                p = leave(lim, rest, r, p, true);
+                p = leave(lim, rest, r, p);
             }
-            s.exit[kThreads - 1] = p;
+            s.tile_exit = p;
         });
         each_free([&](uint32_t t) {
             if (t >= f) entry[t] = (s.entered[t / 32] >> (t % 32)) & 1 ? s.entry[t] : kExitEnd;
         });
     }
 
-    // ---- 2.-5. the tile's tokens: their positions in s.u.e.pos, their count,
-    // and the tile's exit (absolute; kStepEnd when the chain ends).
-    CDB_HD uint32_t find_tokens(uint64_t* exit) {
-        const uint32_t lim = staged_lim();
-        const uint64_t left = S - e;
-        const uint32_t rest = left < kExitMax ? static_cast<uint32_t>(left) : kExitMax - 1;
-        steps(lim);
-        LZC_PHASE(1);
-        Priv<uint32_t> entry, next;
+    // The regions' entries and the tile's exit by rounds of neighbours.
+    CDB_HD void settle(uint32_t lim, uint32_t rest, Priv<uint32_t>& entry) {
+        Priv<uint32_t> next;
         each([&](uint32_t t) {
-            exits(t);
             entry[t] = t * kReg;
-            s.exit[t] = leave(lim, rest, t, t * kReg, t == 0);
+            s.exit[t] = leave_if_sure(lim, rest, t, t * kReg, t == 0);
         });
         for (uint32_t round = 0;; ++round) {
             LZC_EVENT(2, 1);
@@ -743,11 +759,15 @@ struct Chunk {
             uint32_t f = kThreads;  // the first region that is not settled
             for (uint32_t w = kWarps; w-- > 0;)
                 if (s.votes[w]) f = 32 * w + ctz64(s.votes[w]);
-            if (f == kThreads) break;
+            if (f == kThreads) {
+                each([&](uint32_t t) {
+                    if (t == kThreads - 1) s.tile_exit = s.exit[t];
+                });
+                return;
+            }
             const uint32_t sure = f ? s.exit[f - 1] : 0;
             if (round == kRounds) {
-                finish(lim, rest, f, sure, entry);
-                break;
+                return finish(lim, rest, f, sure, entry);
             }
             each([&](uint32_t t) {
                 const uint32_t hi = (t + 1) * kReg;
@@ -759,11 +779,94 @@ struct Chunk {
                     if (p == entry[t]) return;
                 }
                 entry[t] = p;
-                s.exit[t] = p < hi ? leave(lim, rest, t, p, t == f) : p;
+                s.exit[t] = p < hi ? leave_if_sure(lim, rest, t, p, t == f) : p;
             });
         }
+    }
+
+    // The chain from position t % 32 of its warp's regions to past them. Where
+    // a region's exit is not noted, by the format's steps in the staged bytes
+    // (merged lanes take them together).
+    CDB_HD void follow(uint32_t lim, uint32_t rest, uint32_t t) {
+        constexpr uint32_t kSpan = 32 * kReg;  // positions of a warp
+        const uint8_t* step = reinterpret_cast<const uint8_t*>(s.u.w.step);
+        const uint8_t* ex = reinterpret_cast<const uint8_t*>(s.u.w.exit);
+        const Staged in{s.in[buf], staged_at()};
+        const uint32_t lane = t % 32, lo = t / 32 * kSpan, hi = lo + kSpan;
+        uint32_t p = lo + lane;
+        while (p < hi) {
+            if (lane == 0) s.entry[p / kReg] = p;
+            const uint32_t d = ex[p];
+            if (d != kStepSlow) {
+                p += d;
+                continue;
+            }
+            const uint32_t end = (p / kReg + 1) * kReg;
+            while (p < end) {
+                const uint32_t h = step[p];
+                p = h != kStepSlow ? p + h : F::hop_rel(in, p, lim, rest);
+                if (p == kSlowRel) p = kExitOpen;
+            }
+        }
+        s.exit[t] = p;
+    }
+
+    // The tile's chain from warp to warp (one thread).
+    CDB_HD void chase(uint32_t lim, uint32_t rest) {
+        constexpr uint32_t kSpan = 32 * kReg;
+        uint32_t p = 0;
+        for (uint32_t w = 0; w < kWarps; ++w) {
+            const uint32_t lo = w * kSpan, hi = lo + kSpan;
+            s.entered[w] = p;
+            if (p >= hi) continue;
+            uint32_t to = p - lo < 32 ? s.exit[32 * w + p - lo] : kExitOpen;
+            while (to == kExitOpen && p < hi) {
+                LZC_EVENT(2, 1);
+                const uint32_t r = p / kReg;
+                if (s.entry[r] == p) to = s.exit[32 * w];
+                if (to == kExitOpen) p = leave(lim, rest, r, p);
+            }
+            if (to != kExitOpen) p = to;
+        }
+        s.tile_exit = p;
+    }
+
+    // Where the tile's chain enters region t (past it: it does not).
+    CDB_HD uint32_t enter(uint32_t lim, uint32_t rest, uint32_t t) const {
+        uint32_t p = s.entered[t / 32];
+        while (p < t * kReg) {
+            const uint32_t r = p / kReg;
+            if (s.entry[r] == p && s.exit[t & ~31u] != kExitOpen) return s.entry[t];
+            p = leave(lim, rest, r, p);
+        }
+        return p;
+    }
+
+    // ---- 2.-5. the tile's tokens: their positions in s.u.e.pos, their count,
+    // and the tile's exit (absolute; kStepEnd when the chain ends).
+    CDB_HD uint32_t find_tokens(uint64_t* exit) {
+        const uint32_t lim = staged_lim();
+        const uint64_t left = S - e;
+        const uint32_t rest = left < kExitMax ? static_cast<uint32_t>(left) : kExitMax - 1;
+        steps(lim);
+        LZC_PHASE(1);
+        Priv<uint32_t> entry;
+        if constexpr (kThreads <= kSettle) {
+            each_free([&](uint32_t t) { exits(t); });
+            settle(lim, rest, entry);
+        } else {
+            each([&](uint32_t t) {
+                exits(t);
+                s.entry[t] = kExitEnd;
+            });
+            each([&](uint32_t t) { follow(lim, rest, t); });
+            each([&](uint32_t t) {
+                if (t == 0) chase(lim, rest);
+            });
+            each_free([&](uint32_t t) { entry[t] = enter(lim, rest, t); });
+        }
         LZC_PHASE(2);
-        const uint32_t x = s.exit[kThreads - 1];
+        const uint32_t x = s.tile_exit;
         *exit = x == kExitEnd ? kStepEnd : x == kExitFar ? s.far : e + x;
         if (*exit < S) stage(*exit, buf ^ 1);  // lands while this tile's tokens run
         Priv<uint64_t> mask;

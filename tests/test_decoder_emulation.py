@@ -36,8 +36,9 @@ def _build(name):
         os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
     if not os.path.exists(so) or any(os.path.getmtime(d) > os.path.getmtime(so) for d in deps):
         subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-w",
-                        "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, src, "-o", so],
-                       check=True)
+                        "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, src,
+                        "-o", so + ".%d" % os.getpid()], check=True)
+        os.replace(so + ".%d" % os.getpid(), so)  # whole, for workers that build at once
     return ctypes.CDLL(so)
 
 
