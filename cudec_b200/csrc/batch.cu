@@ -38,7 +38,9 @@ std::atomic<int> g_sm_count[kMaxDevices];
 // per batch of 64 KiB LZ4 chunks with 512 / 256 / 128 threads on 148 SMs: 148
 // chunks 174 / 201 / 300, 300 chunks 330 / 216 / 312, 440 chunks 387 / 234 /
 // 337, 592 chunks 527 / 393 / 357, 1,024 chunks 856 / 563 / 447; 16 chunks of
-// 4 MiB 9,550 / 11,720 / 15,980.
+// 4 MiB 9,550 / 11,720 / 15,980. (Taken before wide CTAs chased their chain and
+// the copy was shortened; the chosen widths now take 136, 217 for 440 chunks,
+// 333, 410 and 6,050.)
 constexpr size_t kWideMax = 1, kMediumMax = 3;
 constexpr uint32_t kWideThreads = 256;  // beside narrow CTAs
 // Up to here a wide CTA reads every capacity (148 x 1 MiB out of L2, some 30 us
