@@ -30,9 +30,14 @@
 //   kBarItem   warps 0, 2-5: item i is in its buffer (two buffers in turn,
 //              so warp 0 is at most one item ahead);
 //   kBarReady  (2, by the block's parity) warp 1 arrives, warps 2-5 wait:
-//              the block's literals are in the slot;
+//              the block's literals are in the slot, or the block is faulty;
 //   kBarFree   (2) warps 2-5 arrive, warp 1 waits: the block is executed;
 //   kBarExec   warps 2-5.
+// Warp 1 arrives at a block's kBarReady only after its wait at the kBarFree of
+// the block two before, which the block's own kBarFree shares: so warps 2-5
+// wait at the kBarReady of every block that they begin, a faulty one
+// included, before they arrive at its kBarFree. Without that a warp 1 that is
+// late would be overtaken at that barrier and the CTA would not end.
 // A fault found by warp 0 travels as an item, one found by warp 1 as the
 // block's literal fault, so that warps 2-5 meet everything in the serial
 // decoder's order and alone decide the frame's status. The one that ends the
@@ -898,16 +903,18 @@ struct ExecRole {
             const Item it = s.item[i & 1];
             int st = CUDEC_OK;   // ends the frame here
             bool over = false;   // warp 0 makes no further item
+            if (it.flags & kFirst) {
+                ZS_T(t1);
+                bar_sync(kBarReady + static_cast<int>(block & 1), kLitCount);
+                ZS_ADD(6, t1);
+                ++waited;
+            }
             if (it.kind == kFault) {
                 st = CUDEC_ERR_CORRUPT_INPUT;
                 over = true;
             } else {
                 over = (it.flags & kEnd) != 0;
                 if (it.flags & kFirst) {
-                    ZS_T(t1);
-                    bar_sync(kBarReady + static_cast<int>(block & 1), kLitCount);
-                    ZS_ADD(6, t1);
-                    ++waited;
                     exec = CUDEC_OK;
                     lp = 0;
                     lit = it.lit != nullptr ? it.lit : slot + s.lit_at[block & 1];

@@ -1,10 +1,13 @@
 // A CUDA CTA on the host, for the CPU tests of device code written with warp
 // collectives and barriers: every thread is a fiber, run one at a time, that
-// gives way where it meets a collective or a barrier. A collective completes
-// when all 32 lanes have reached it, a barrier when its thread count has; if
-// every fiber waits, the CTA has deadlocked and run() returns false. The
-// order in which runnable fibers are taken is drawn from a seed, so that code
-// which leans on an order that CUDA does not give shows it. Test
+// gives way where it meets a collective or a barrier, an arrival without a
+// wait included. A collective completes when all 32 lanes have reached it, a
+// barrier when its thread count has; if every fiber waits, the CTA has
+// deadlocked and run() returns false, as it does where a thread meets a
+// barrier twice before it completes or threads state different counts for it.
+// The order in which runnable fibers are taken is drawn from the seed, and a
+// seed can name a warp that only runs when no other can, so that code which
+// leans on an order or a pace that CUDA does not give shows it. Test
 // infrastructure only.
 #pragma once
 
@@ -30,9 +33,10 @@ namespace emul {
 
 struct Fiber {
     ucontext_t ctx;
-    std::unique_ptr<char[]> stack;
     bool done = false;
-    bool waiting = false;
+    const uint32_t* gen = nullptr;  // what it waits for: *gen to differ from `at`
+    uint32_t at = 0;
+    bool runnable() const { return !done && (gen == nullptr || *gen != at); }
 };
 
 struct Warp {
@@ -42,7 +46,8 @@ struct Warp {
 };
 
 struct Barrier {
-    uint32_t arrived = 0, gen = 0;
+    uint32_t arrived = 0, gen = 0, count = 0;
+    std::vector<uint32_t> seen;  // per thread: 1 + the generation it last arrived in
 };
 
 struct Cta {
@@ -53,7 +58,6 @@ struct Cta {
     Barrier bars[16];
     ucontext_t main_ctx;
     uint32_t cur = 0;
-    uint64_t progress = 0;  // completed collectives, barriers and fibers
     const char* bad = nullptr;
     std::function<void()> body;
 };
@@ -63,21 +67,35 @@ inline Cta*& cta() {
     return c;
 }
 
-inline void give_way() {
+// Back to the scheduler until *gen differs from `at` (null: until its turn).
+inline void give_way(const uint32_t* gen = nullptr, uint32_t at = 0) {
     Cta* c = cta();
-    swapcontext(&c->fibers[c->cur].ctx, &c->main_ctx);
+    Fiber& f = c->fibers[c->cur];
+    f.gen = gen;
+    f.at = at;
+    swapcontext(&f.ctx, &c->main_ctx);
+}
+
+inline void fail(const char* why) {
+    cta()->bad = why;
+    give_way();  // for good
 }
 
 inline void entry() {
     Cta* c = cta();
     c->body();
     c->fibers[c->cur].done = true;
-    ++c->progress;
     swapcontext(&c->fibers[c->cur].ctx, &c->main_ctx);
 }
 
+// The seed whose order is `order` (below 256; 0: by thread number) and that
+// starves warp `warp`.
+constexpr uint64_t starving(uint64_t order, uint32_t warp) {
+    return order | static_cast<uint64_t>(warp + 1) << 8;
+}
+
 // Runs `body` as `threads` threads; false when they deadlock or misuse a
-// collective.
+// collective or a barrier.
 inline bool run(uint32_t threads, uint64_t seed, std::function<void()> body) {
     static std::vector<std::unique_ptr<char[]>> pool;
     static Cta c;
@@ -86,6 +104,7 @@ inline bool run(uint32_t threads, uint64_t seed, std::function<void()> body) {
     c.body = std::move(body);
     c.fibers.resize(threads);
     c.warps.resize(threads / 32);
+    for (Barrier& b : c.bars) b.seen.assign(threads, 0);
     cta() = &c;
     while (pool.size() < threads) pool.emplace_back(new char[Cta::kStack]);
     for (uint32_t t = 0; t < threads; ++t) {
@@ -96,35 +115,31 @@ inline bool run(uint32_t threads, uint64_t seed, std::function<void()> body) {
         f.ctx.uc_link = nullptr;
         makecontext(&f.ctx, entry, 0);
     }
-    uint64_t rng = seed * 0x9E3779B97F4A7C15ull + 1;
+    const uint64_t order = seed & 255;
+    const uint32_t starved = static_cast<uint32_t>(seed >> 8);  // 1 + the warp
+    uint64_t rng = order * 0x9E3779B97F4A7C15ull + 1;
     for (;;) {
-        const uint64_t before = c.progress;
-        uint32_t live = 0;
         rng = rng * 6364136223846793005ull + 1442695040888963407ull;
-        const uint32_t start = seed ? static_cast<uint32_t>(rng >> 33) % threads : 0;
-        const bool down = seed && (rng >> 62 & 1);
-        for (uint32_t k = 0; k < threads; ++k) {
-            const uint32_t t = (start + (down ? threads - k : k)) % threads;
-            if (c.fibers[t].done) continue;
-            ++live;
-            c.cur = t;
-            swapcontext(&c.main_ctx, &c.fibers[t].ctx);
-            if (c.bad) return false;
-        }
-        if (!live) return true;
-        if (c.progress == before) {
-            // one more round: a fiber may have been released by a later one
-            uint64_t b2 = c.progress;
-            for (uint32_t t = 0; t < threads; ++t) {
-                if (c.fibers[t].done) continue;
+        const uint32_t start = order ? static_cast<uint32_t>(rng >> 33) % threads : 0;
+        const bool down = order && (rng >> 62 & 1);
+        bool ran = false;
+        // the starved warp in a turn of its own, when no other thread can run
+        for (int turn = 0; turn < 2 && !ran; ++turn)
+            for (uint32_t k = 0; k < threads; ++k) {
+                const uint32_t t = (start + (down ? threads - k : k)) % threads;
+                if ((turn == 1) != (t / 32 + 1 == starved) || !c.fibers[t].runnable()) continue;
+                ran = true;
                 c.cur = t;
                 swapcontext(&c.main_ctx, &c.fibers[t].ctx);
+                if (c.bad) return false;
             }
-            if (c.progress == b2) {
+        if (ran) continue;
+        for (uint32_t t = 0; t < threads; ++t)
+            if (!c.fibers[t].done) {
                 c.bad = "deadlock";
                 return false;
             }
-        }
+        return true;
     }
 }
 
@@ -134,18 +149,14 @@ inline const uint64_t* collect(int op, uint64_t v) {
     Warp& w = c->warps[c->cur / 32];
     const uint32_t lane = c->cur % 32, gen = w.gen;
     if (w.arrived == 0) w.op = op;
-    if (w.op != op) {
-        c->bad = "lanes of a warp at different collectives";
-        give_way();
-    }
+    if (w.op != op) fail("lanes of a warp at different collectives");
     uint64_t* slot = w.value[gen & 1];
     slot[lane] = v;
     if (++w.arrived == 32) {
         w.arrived = 0;
         ++w.gen;
-        ++c->progress;
     } else {
-        while (w.gen == gen) give_way();
+        give_way(&w.gen, gen);
     }
     return slot;
 }
@@ -154,13 +165,16 @@ inline void bar(int id, uint32_t n, bool wait) {
     Cta* c = cta();
     Barrier& b = c->bars[id];
     const uint32_t gen = b.gen;
+    if (b.arrived != 0 && b.count != n) fail("threads state different counts for a barrier");
+    if (b.seen[c->cur] == gen + 1) fail("a thread meets a barrier twice before it completes");
+    b.count = n;
+    b.seen[c->cur] = gen + 1;
     if (++b.arrived == n) {
         b.arrived = 0;
         ++b.gen;
-        ++c->progress;
-    } else if (wait) {
-        while (b.gen == gen) give_way();
     }
+    if (!wait) give_way();
+    else if (b.gen == gen) give_way(&b.gen, gen);
 }
 
 struct Idx {

@@ -3,7 +3,7 @@
 tests/native/cuda_emul.h runs a CTA's threads as fibers that meet at warp
 collectives and barriers (a deadlock, lanes at different collectives, or
 threads that disagree on the result fail the run), in an order drawn from a
-seed. The sizes are those where the decoders change their way: LZ4 and Snappy
+seed, or with one warp held back until no other can run. The sizes are those where the decoders change their way: LZ4 and Snappy
 chunks of one tile and of several at each width of the CTA, batches cut by
 long tokens, tiles that few tokens settle; Zstd frames of no, one and more
 than one item of 128 sequences, one and several blocks, literal streams shared
@@ -168,6 +168,53 @@ def test_zstd_mutants(zstd):
         if k % 5 == 0:
             two = f + b"\x50\x2a\x4d\x18\x03\x00\x00\x00abc" + mutate(rng, frames[0][0])
             check(zstd["multi"], oracle.zstd_decode_multi, two, 2 * cap, k, 0, ("multi", k))
+
+
+def block(kind, body, size=None, last=False):
+    n = len(body) if size is None else size
+    return (n << 3 | kind << 1 | last).to_bytes(3, "little") + body
+
+
+RAW, RLE, COMPRESSED, RESERVED = range(4)
+# blocks that decode, of few bytes or none
+SMALL = [block(RAW, b"abcd"), block(RAW, b""), block(RLE, b"x", 9), block(RLE, b"x", 0),
+         block(COMPRESSED, b"\x18abc\x00")]  # three raw literals, no sequences
+# blocks that do not, by the part of the decoder that finds it
+FAULTY = {
+    "reserved type": block(RESERVED, b""),
+    "past the frame": block(RAW, b"ab", 70),
+    "no header": b"",
+    "no literals header": block(COMPRESSED, b""),
+    "literals past the block": block(COMPRESSED, b"\x28ab"),
+    "no sequences header": block(COMPRESSED, b"\x18abc"),
+    "literals without a table": block(COMPRESSED, b"\x43\xc0\x00zzz\x00"),
+    "literals with a bad table": block(COMPRESSED, b"\x42\xc0\x00\xff\x00\x00\x00"),
+    "reserved modes": block(COMPRESSED, b"\x18abc\x01\x03\x80"),
+    "no sequence table to repeat": block(COMPRESSED, b"\x18abc\x01\xfc\x80"),
+    "a code past the last": block(COMPRESSED, b"\x18abc\x01\x40\x3f\x80"),
+    "no bitstream": block(COMPRESSED, b"\x18abc\x01\x00"),
+    "no padding marker": block(COMPRESSED, b"\x18abc\x01\x00\x00"),
+    "bitstream over-read": block(COMPRESSED, b"\x18abc\x01\x00\xff\xff\x07"),
+    "an offset past the output": block(COMPRESSED, b"\x18abc\x01\x54\x03\x1f\x00" + b"\xff" * 4),
+}
+
+
+# A fault that ends the frame in its first, second or a later block, with each
+# of the six warps as far behind the others as their barriers let it be.
+@pytest.mark.parametrize("fault", FAULTY)
+def test_zstd_faulty_block(zstd, fault):
+    rng = random.Random(fault)
+    head = b"\x28\xb5\x2f\xfd\xa0" + (64).to_bytes(4, "little")
+    for before in range(4):
+        for _ in range(2):
+            f = head + b"".join(rng.choice(SMALL) for _ in range(before)) + FAULTY[fault]
+            if fault != "no header" and rng.random() < 0.5:
+                f += rng.choice(SMALL)
+            assert oracle.zstd_decode(f, 64)[0] == 2
+            for warp in range(6):
+                seed = rng.randrange(256) | (warp + 1) << 8
+                check(zstd["one"], oracle.zstd_decode, f, 64, seed, 0, (f, warp))
+                check(zstd["multi"], oracle.zstd_decode_multi, f, 64, seed, 0, (f, warp))
 
 
 @pytest.mark.parametrize("size", [0, 1, 63, 3000, 20000, 65536])
