@@ -80,6 +80,25 @@ def gdeflate():
     return lib.gdeflate_emulate
 
 
+def starving(order, warp):
+    """The seed of order `order` that holds warp `warp` back."""
+    return order | (warp + 1) << 8
+
+
+# What the checks above rest on: two warps of code with a barrier each way.
+@pytest.mark.parametrize("kind,why", [
+    (0, None), (1, "a thread meets a barrier twice before it completes"),
+    (2, "threads state different counts for a barrier"), (3, "deadlock"),
+    (4, "lanes of a warp at different collectives")])
+def test_emulation(kind, why):
+    lib = _build("emul_check")
+    lib.emul_check.restype = ctypes.c_char_p
+    lib.emul_check.argtypes = [ctypes.c_int, ctypes.c_uint64]
+    found = {lib.emul_check(kind, seed) for order in range(8)
+             for seed in (order, starving(order, 0), starving(order, 1))}
+    assert found == {None} if why is None else why.encode() in found
+
+
 def check(run, want, comp, cap, seed=0, skew=0, label=None):
     src = np.zeros(len(comp) + 64 + skew, dtype=np.uint8)
     src[32 + skew:32 + skew + len(comp)] = np.frombuffer(comp, dtype=np.uint8)
@@ -139,10 +158,12 @@ def test_lz(lz, size, threads):
         for fmt, pack, want in ((0, W.lz4_compress, oracle.lz4_decode),
                                 (1, W.snappy_compress, oracle.snappy_decode)):
             f = pack(data)
-            check(lz(fmt, threads), want, f, size, k + 1, (5 * k + fmt) % 16, (size, k, fmt))
+            late = rng.randrange(threads // 32)
+            check(lz(fmt, threads), want, f, size, starving(k + 1, late), (5 * k + fmt) % 16,
+                  (size, k, fmt))
             for m in range(4 if size < 6000 else 1):
-                check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2, m, 0,
-                      (size, k, fmt, m))
+                check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2,
+                      starving(m, late) if m % 2 else m, 0, (size, k, fmt, m))
 
 
 @pytest.mark.parametrize("size", [0, 1, 40, 1000, 1600, 9000, 131072, 150000])
@@ -150,7 +171,8 @@ def test_zstd(zstd, size):
     for k, data in enumerate(contents(size)):
         for level in (1, 19):
             f = W.zstd_compress(data, level, 20, level == 19)
-            check(zstd["one"], oracle.zstd_decode, f, size, k, (5 * k + level) % 16,
+            check(zstd["one"], oracle.zstd_decode, f, size,
+                  starving(k, (k + size) % 6) if level == 1 else k, (5 * k + level) % 16,
                   (size, k, level))
     check(zstd["one"], oracle.zstd_decode, f, size + 9, 3, 1, (size, "room"))
 
@@ -164,10 +186,11 @@ def test_zstd_mutants(zstd):
         if cap > 100000 and k % 3:
             continue
         cut = rng.choice([0, 0, 1, cap // 2])
-        check(zstd["one"], oracle.zstd_decode, mutate(rng, f), cap - cut, k, k % 16, k)
+        seed = starving(k, rng.randrange(6))
+        check(zstd["one"], oracle.zstd_decode, mutate(rng, f), cap - cut, seed, k % 16, k)
         if k % 5 == 0:
             two = f + b"\x50\x2a\x4d\x18\x03\x00\x00\x00abc" + mutate(rng, frames[0][0])
-            check(zstd["multi"], oracle.zstd_decode_multi, two, 2 * cap, k, 0, ("multi", k))
+            check(zstd["multi"], oracle.zstd_decode_multi, two, 2 * cap, seed, 0, ("multi", k))
 
 
 def block(kind, body, size=None, last=False):
@@ -212,7 +235,7 @@ def test_zstd_faulty_block(zstd, fault):
                 f += rng.choice(SMALL)
             assert oracle.zstd_decode(f, 64)[0] == 2
             for warp in range(6):
-                seed = rng.randrange(256) | (warp + 1) << 8
+                seed = starving(rng.randrange(256), warp)
                 check(zstd["one"], oracle.zstd_decode, f, 64, seed, 0, (f, warp))
                 check(zstd["multi"], oracle.zstd_decode_multi, f, 64, seed, 0, (f, warp))
 
