@@ -1132,57 +1132,119 @@ struct Chunk {
 };
 
 // ---------------------------------------------------------------------------
-// The batch kernels. Dynamic shared memory: sizeof(Shm).
-#if defined(__CUDACC__)
-// In a batch of many chunks a few large ones would run on alone at the
-// narrow CTAs' pace: those are left to a CTA each of the wide kernel that runs
-// beside. Large: a capacity of 2^k bytes or more, for the smallest k from
-// kLargeLog on that leaves no more of them than the wide kernel has CTAs (a
-// batch of many large chunks has the SMs busy to its end anyway). Measured:
+// A batch's large chunks. In a batch of many chunks a few large ones would run
+// on alone at the narrow CTAs' pace: those are left to a CTA each of the wide
+// kernel that runs beside. Large: a capacity of 2^k bytes or more, for the
+// smallest k from kLargeLog on that leaves no more of them than the wide kernel
+// has CTAs (a batch of many large chunks has the SMs busy to its end anyway).
+// Measured:
 // 8,000 uneven Snappy chunks (256 bytes to 4 MiB, median 16 KiB) 7,997 us
 // without the wide kernel, 4,950 with it; 2,000 of them 4,084 and 2,610;
 // 30,000 uneven LZ4 chunks 5,901 and 3,811, with kLargeLog 19 4,022, with 17
-// the same. Where no chunk is large the count of them costs 2 us in 410
-// (1,024 chunks) to 8 in 443 (8,192).
+// the same.
+//
+// `Caps` is the batch's capacities (the CPU tests count the reads).
+#if defined(__CUDACC__) || defined(CDB_EMULATE)
 constexpr uint32_t kLargeLog = 18, kLogs = 16;
 
-// The k - kLargeLog of the batch (kLogs: no chunk is large), by the whole CTA;
-// count: the large chunks.
-__device__ __forceinline__ uint32_t large_from(const size_t* caps, size_t n, uint32_t wide,
+// Size class of a capacity: 0 below 2^kLargeLog, then one per power of two up
+// to kLogs.
+__device__ __forceinline__ uint32_t large_class(uint64_t cap) {
+    const uint64_t c = cap >> kLargeLog;
+    const uint32_t k = c ? 64 - __clzll(static_cast<long long>(c)) : 0;
+    return k < kLogs ? k : kLogs;
+}
+// Whether a capacity is of class k (1 or more) or a higher one.
+__device__ __forceinline__ bool from_class(uint64_t cap, uint32_t k) {
+    return (cap >> (kLargeLog + k - 1)) != 0;
+}
+
+// The class from which on the batch's chunks are large (above kLogs: none is),
+// by the whole CTA of T threads; count: the large chunks. A warp adds the
+// chunks of a class in one go: a batch's capacities are often all alike.
+template <uint32_t T, class Caps>
+__device__ __forceinline__ uint32_t large_from(const Caps& caps, size_t n, uint32_t wide,
                                                uint32_t* count) {
-    __shared__ uint32_t hist[kLogs];
-    if (threadIdx.x < kLogs) hist[threadIdx.x] = 0;
+    __shared__ uint32_t hist[kLogs + 1];
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    if (t <= kLogs) hist[t] = 0;
     __syncthreads();
-#pragma unroll 8
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint64_t c = caps[i];
-        if (c >> kLargeLog) {
-            const uint32_t k = 63 - kLargeLog - __clzll(static_cast<long long>(c));
-            atomicAdd(&hist[k < kLogs ? k : kLogs - 1], 1u);
+    constexpr uint32_t U = 8;
+    for (size_t i0 = 0; i0 < n; i0 += T * U) {
+        uint64_t c[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const size_t i = i0 + u * T + t;
+            c[u] = i < n ? caps[i] : 0;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            if (!__any_sync(0xffffffffu, (c[u] >> kLargeLog) != 0)) continue;
+            const uint32_t k = large_class(c[u]);
+            const unsigned same = __match_any_sync(0xffffffffu, k);
+            if ((same >> lane) == 1u) atomicAdd(&hist[k], __popc(same));
         }
     }
     __syncthreads();
-    uint32_t k = kLogs, sum = 0;
-    while (k != 0 && hist[k - 1] <= wide - sum) sum += hist[--k];
+    uint32_t k = kLogs + 1, sum = 0;
+    while (k > 1 && hist[k - 1] <= wide - sum) sum += hist[--k];
     __syncthreads();  // read by every thread before the next use
     *count = sum;
-    return sum ? k : kLogs;
-}
-__device__ __forceinline__ bool is_large(uint64_t cap, uint32_t k) {
-    return k < kLogs && (cap >> (kLargeLog + k)) != 0;
+    return sum ? k : kLogs + 1;
 }
 
-// The index of the batch's large chunk number w (threads' shares in turn), by
-// the whole CTA of T threads; w < their count.
-template <uint32_t T>
-__device__ __forceinline__ size_t large_chunk(const size_t* caps, size_t n, uint32_t k,
+// Whether chunk c (of class 1 or more) is one of the large ones, by the whole
+// CTA of T threads: at most `wide` chunks are of its class or a higher one.
+// The chunks are read from c on, round the end, until more than `wide` of them
+// are known, at first 2 per thread between barriers, then twice as many each
+// time. So all the calls of a launch for one class read no more than some
+// 2 (wide + 1) n capacities together, wherever its chunks lie in the batch, and
+// 2 T each where all capacities are alike. Us for LZ4 pages of 4 KiB in slots of
+// 1 MiB, when each narrow CTA counted the whole batch, and now; in slots of
+// 4 KiB: 8,192 pages 434, 329; 319. 100,000 pages 19,558, 3,781; 3,610.
+template <uint32_t T, class Caps>
+__device__ __forceinline__ bool is_large(const Caps& caps, size_t n, uint32_t wide, size_t c) {
+    __shared__ uint32_t found;
+    const uint32_t t = threadIdx.x, lane = t & 31;
+    if (t == 0) found = 0;
+    __syncthreads();
+    const uint32_t k = large_class(caps[c]);
+    uint32_t seen = 0;
+    constexpr uint32_t U = 2, kMost = 16;
+    uint32_t per = U;
+    for (size_t at = 0; at < n && seen <= wide; at += static_cast<size_t>(T) * per) {
+        if (at != 0 && per < kMost) per *= 2;
+        uint32_t mine = 0;
+        for (uint32_t u0 = 0; u0 < per; u0 += U) {
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const size_t q = at + (u0 + u) * T + t;
+                size_t i = c + q;
+                if (i >= n) i -= n;
+                mine += q < n && from_class(caps[i], k);
+            }
+        }
+#pragma unroll
+        for (uint32_t d = 16; d; d >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, d);
+        if (lane == 0 && mine) atomicAdd(&found, mine);
+        __syncthreads();
+        seen = found;
+        __syncthreads();  // read by every thread before the next addition
+    }
+    return seen <= wide;
+}
+
+// The index of chunk number w of class k or higher (threads' shares in turn),
+// by the whole CTA of T threads; w < their count.
+template <uint32_t T, class Caps>
+__device__ __forceinline__ size_t large_chunk(const Caps& caps, size_t n, uint32_t k,
                                               uint32_t w) {
     __shared__ uint32_t sums[T / 32];
     __shared__ size_t found;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     uint32_t mine = 0;
 #pragma unroll 4
-    for (size_t i = t; i < n; i += T) mine += is_large(caps[i], k);
+    for (size_t i = t; i < n; i += T) mine += from_class(caps[i], k);
     uint32_t before = mine;  // then inclusive over the warp
 #pragma unroll
     for (uint32_t d = 1; d < 32; d <<= 1) {
@@ -1195,13 +1257,17 @@ __device__ __forceinline__ size_t large_chunk(const size_t* caps, size_t n, uint
     if (w < before && w >= before - mine) {
         uint32_t left = w - (before - mine);
         size_t i = t;
-        while (!is_large(caps[i], k) || left-- != 0) i += T;
+        while (!from_class(caps[i], k) || left-- != 0) i += T;
         found = i;
     }
     __syncthreads();
     return found;
 }
+#endif
 
+// ---------------------------------------------------------------------------
+// The batch kernels. Dynamic shared memory: sizeof(Shm).
+#if defined(__CUDACC__)
 template <class F, uint32_t kThreads>
 __device__ __forceinline__ void decode_chunk(size_t c, const void* const* src_ptrs,
                                              const size_t* src_sizes, void* const* dst_ptrs,
@@ -1225,10 +1291,8 @@ template <class F, uint32_t kThreads>
 __global__ void __launch_bounds__(kThreads, Width<kThreads>::kPerSm)
     lz_cta_kernel(const void* const* src_ptrs, const size_t* src_sizes, void* const* dst_ptrs,
                   const size_t* dst_caps, size_t n, cudec_chunk_result* results, uint32_t wide) {
-    uint32_t count;
     for (size_t c = blockIdx.x; c < n; c += gridDim.x) {
-        if (wide && (dst_caps[c] >> kLargeLog) &&
-            is_large(dst_caps[c], large_from(dst_caps, n, wide, &count)))
+        if (wide && large_class(dst_caps[c]) && is_large<kThreads>(dst_caps, n, wide, c))
             continue;  // a wide CTA's
         decode_chunk<F, kThreads>(c, src_ptrs, src_sizes, dst_ptrs, dst_caps, results);
     }
@@ -1242,7 +1306,7 @@ __global__ void __launch_bounds__(kThreads, Width<kThreads>::kPerSm)
     lz_wide_kernel(const void* const* src_ptrs, const size_t* src_sizes, void* const* dst_ptrs,
                    const size_t* dst_caps, size_t n, cudec_chunk_result* results) {
     uint32_t count;
-    const uint32_t k = large_from(dst_caps, n, gridDim.x, &count);
+    const uint32_t k = large_from<kThreads>(dst_caps, n, gridDim.x, &count);
     // a CTA without work leaves first, so that the narrow ones spread evenly
     if (blockIdx.x >= count) return;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -28,6 +28,7 @@
 #define __noinline__ inline
 #define __constant__
 #define __align__(n) alignas(n)
+#define __shared__ static
 
 namespace emul {
 
@@ -231,6 +232,7 @@ inline unsigned __match_any_sync(unsigned, uint32_t x) {
 }
 inline float __fdividef(float a, float b) { return a / b; }
 inline int __clz(uint32_t x) { return x ? __builtin_clz(x) : 32; }
+inline int __clzll(long long x) { return x ? __builtin_clzll(static_cast<uint64_t>(x)) : 64; }
 inline int __ffs(uint32_t x) { return __builtin_ffs(static_cast<int>(x)); }
 inline int __ffsll(long long x) { return __builtin_ffsll(x); }
 inline int __popc(uint32_t x) { return __builtin_popcount(x); }
@@ -257,6 +259,11 @@ T __ldg(const T* p) {
     return *p;
 }
 
+inline uint32_t atomicAdd(uint32_t* a, uint32_t v) {
+    const uint32_t old = *a;
+    *a += v;
+    return old;
+}
 inline uint32_t atomicOr(uint32_t* a, uint32_t v) {
     const uint32_t old = *a;
     *a |= v;

@@ -37,7 +37,49 @@ int widths(uint32_t threads, const uint8_t* src, uint64_t S, uint8_t* dst, uint6
                             : run<F, 512>(src, S, dst, cap, seed, written);
 }
 
+// A batch's capacities, their reads counted.
+struct Caps {
+    const size_t* p;
+    size_t n;
+    uint64_t* reads;
+    size_t operator[](size_t i) const {
+        if (i >= n) std::abort();
+        ++*reads;
+        return p[i];
+    }
+};
+
 }  // namespace
+
+// The large chunks of a batch, as the wide kernel's `wide` CTAs pick them
+// (chunk[0, *count): its index, one per CTA) and as the narrow CTAs of the m
+// chunks at `ask` find them (is[0, m)); reads: capacities that those m read.
+// -1: the CTA deadlocks.
+extern "C" int lz_large(const size_t* caps, size_t n, uint32_t wide, uint64_t seed,
+                        uint64_t* chunk, uint32_t* count, const uint64_t* ask, size_t m,
+                        uint8_t* is, uint64_t* reads) {
+    uint64_t other = 0;
+    *reads = 0;
+    const Caps w{caps, n, &other}, c{caps, n, reads};
+    if (!emul::run(256, seed, [&] {
+            uint32_t cnt = 0;
+            const uint32_t k = cdb::lzc::large_from<256>(w, n, wide, &cnt);
+            if (threadIdx.x == 0) *count = cnt;
+            for (uint32_t i = 0; i < cnt; ++i) {
+                const size_t at = cdb::lzc::large_chunk<256>(w, n, k, i);
+                __syncthreads();
+                if (threadIdx.x == 0) chunk[i] = at;
+            }
+        }))
+        return -1;
+    const bool ok = emul::run(128, seed, [&] {
+        for (size_t i = 0; i < m; ++i) {
+            const bool large = cdb::lzc::is_large<128>(c, n, wide, ask[i]);
+            if (threadIdx.x == 0) is[i] = large;
+        }
+    });
+    return ok ? 0 : -1;
+}
 
 // fmt 0 = LZ4, 1 = Snappy; -1: the CTA deadlocks or its lanes meet different
 // collectives.

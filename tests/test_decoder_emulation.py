@@ -48,10 +48,14 @@ def lz():
     lib.lz_emulate.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_uint64,
                                ctypes.c_void_p, ctypes.c_uint64, ctypes.c_uint64,
                                ctypes.POINTER(ctypes.c_uint64)]
+    lib.lz_large.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint32, ctypes.c_uint64,
+                             ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t,
+                             ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)]
 
     def call(fmt, threads):
         return lambda src, n, dst, cap, seed, written: lib.lz_emulate(
             fmt, threads, src, n, dst, cap, seed, written)
+    call.lib = lib
     return call
 
 
@@ -164,6 +168,49 @@ def test_lz(lz, size, threads):
             for m in range(4 if size < 6000 else 1):
                 check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2,
                       starving(m, late) if m % 2 else m, 0, (size, k, fmt, m))
+
+
+def capacities(kind, n):
+    rng = random.Random(kind)
+    if kind == "alike":
+        return [1 << 20] * n
+    if kind == "none":
+        return [(1 << 18) - 1] * n
+    if kind == "at the end":
+        return [4096] * (n - n // 2) + [1 << 18] * (n // 2)
+    if kind == "few":
+        return [rng.choice([1 << 18, 1 << 40, 2**64 - 1]) if i % 211 == 5 else 100
+                for i in range(n)]
+    return [int(2 ** rng.uniform(10, 23 if kind == "uneven" else 45)) for _ in range(n)]
+
+
+# Which chunks of a batch a wide CTA takes: those of a size class that holds,
+# with the ones above it, no more of them than there are wide CTAs. The wide
+# and the narrow CTAs come to the same answer, and the narrow ones read a
+# bounded number of capacities for it, not the batch's for each chunk.
+@pytest.mark.parametrize("kind", ["alike", "none", "at the end", "few", "uneven", "very uneven"])
+@pytest.mark.parametrize("n,wide", [(445, 148), (2000, 148), (2000, 5)])
+def test_lz_large_chunks(lz, kind, n, wide):
+    caps = capacities(kind, n)
+    level = [min(max(c.bit_length() - 18, 0), 16) for c in caps]
+    first = next((k for k in range(1, 17) if sum(v >= k for v in level) <= wide), 17)
+    want = [i for i in range(n) if level[i] >= first]
+    arr = np.array(caps, dtype=np.uint64)
+    ask = [i for i in range(n) if level[i]]
+    if len(ask) > 150:  # every large one among them
+        ask = sorted(set(random.Random(n).sample(ask, 150)) | set(want))
+    ask = np.array(ask, dtype=np.uint64)
+    chunk = np.zeros(wide, dtype=np.uint64)
+    count, reads = ctypes.c_uint32(0), ctypes.c_uint64(0)
+    large = np.zeros(max(len(ask), 1), dtype=np.uint8)
+    assert lz.lib.lz_large(arr.ctypes.data, n, wide, starving(n % 250, wide % 4),
+                           chunk.ctypes.data, ctypes.addressof(count), ask.ctypes.data, len(ask),
+                           large.ctypes.data, ctypes.byref(reads)) == 0
+    assert sorted(chunk[:count.value].tolist()) == want
+    assert [int(i) for i, v in zip(ask, large) if v] == want
+    # the CTA's first step and the chunk's own capacity, then what a class reads together
+    together = 0 if kind == "alike" else 2 * (wide + 1) * n * len(set(level))
+    assert reads.value <= 3 * 128 * len(ask) + together
 
 
 @pytest.mark.parametrize("size", [0, 1, 40, 1000, 1600, 9000, 131072, 150000])

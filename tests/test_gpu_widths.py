@@ -114,3 +114,21 @@ def test_large_among_many_captured(cuda):
     assert (b.results()["status"] == 0).all()
     for i, r in enumerate(raws):
         assert b.output(i, dst) == r, i
+
+
+@pytest.mark.parametrize("fmt", ["lz4", "snappy"])
+def test_generous_capacities(cuda, fmt):
+    """Small pages in slots of 256 KiB: none of so many is large."""
+    import torch
+    n = 1500
+    raws = [r[:2000 + i % 999] for i, r in enumerate(chunks(n))]
+    comps = [PACK[fmt](r) for r in raws]
+    b = DeviceBatch(comps, [262144] * n, device=cuda, dst_align=16, dst_skew=3, src_skew=5)
+    assert b.run(fmt) == 0
+    torch.cuda.synchronize()
+    res = b.results()
+    assert (res["status"] == 0).all()
+    assert [int(v) for v in res["bytes_written"]] == [len(r) for r in raws]
+    dst = b.dst_host()
+    for i, r in enumerate(raws):
+        assert b.output(i, dst, len(r) + 64) == r + b"\xa5" * 64, i
