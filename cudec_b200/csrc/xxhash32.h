@@ -42,6 +42,10 @@ class Xxh32 {
             c = xxh_rotl(c + xxh_read32(p + 8) * kXxhP2, 13) * kXxhP1;
             d = xxh_rotl(d + xxh_read32(p + 12) * kXxhP2, 13) * kXxhP1;
         }
+        // One register each: seen as one vector (they leave for one array), the
+        // four took 32-bit vector products without hardware for them, 2.5 GB/s
+        // instead of 5.1.
+        asm("" : "+r"(a), "+r"(b), "+r"(c), "+r"(d));
         v_[0] = a, v_[1] = b, v_[2] = c, v_[3] = d;
     }
 
