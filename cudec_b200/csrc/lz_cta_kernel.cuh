@@ -51,7 +51,12 @@
 //      taken modulo its length, so a match costs one hop) until a literal
 //      or a byte before the window is met, so no byte waits for another.
 //      A token longer than kBig is copied by the whole CTA, 16 bytes per
-//      thread at a time.
+//      thread at a time: an LZ4 one in its place between the batch's other
+//      tokens, whose parse still holds; Snappy's (literals, and rare) and those
+//      that only the ladder can read end the batch. When each ended it, and a
+//      match from less than 16 bytes per thread back was always written from
+//      its period, 100 chunks of 64 KiB of matches of 1,100 to 4,000 bytes took
+//      269 us, 16 of 4 MiB 12,816; now 119 and 4,443.
 //
 // What bounds it: instruction issue (77 % of the issue slots at seven CTAs per
 // SM; 290,000 warp instructions per 64 KiB chunk of 5,250 tokens, two thirds
@@ -175,6 +180,12 @@ __device__ unsigned long long lzc_events[16];
 #define LZC_START() \
     do {            \
     } while (0)
+#endif
+
+#if defined(__CUDACC__)
+#define LZC_APART __host__ __device__ __noinline__
+#else
+#define LZC_APART inline
 #endif
 
 // ---------------------------------------------------------------------------
@@ -493,11 +504,14 @@ struct SnappyF : lzl::SnappyLadder {
 };
 
 // ---------------------------------------------------------------------------
-// What ends a batch early: the first failing or terminal token, the first
-// token that the whole CTA copies.
+// What ends a batch early, its first event: a failing or terminal token, or one
+// whose lengths only the ladder tells. And the batch's first long token.
 struct Cut {
     uint32_t event, big;
 };
+// An event token's code: its status when it fails, or
+constexpr int32_t kEnd = CUDEC_OK;    // terminal, executed with the batch
+constexpr int32_t kFar = INT32_MIN;   // copied by exec_far()
 
 // Shared memory of one CTA. The input is staged in two buffers in turn: the
 // next tile's bytes land while this one's tokens run.
@@ -515,18 +529,19 @@ struct Shm : Width<kThreads> {
             Rec rec[kThreads];
             Sector map[kSectors];
             uint16_t pos[kMaxTok];   // the tile's tokens, relative to its entry
+            uint8_t period[16 * kThreads];  // whole-CTA copies: a short match's period
         } e;
-        uint8_t period[16 * kThreads];  // whole-CTA copies: a short match's period
     } u;
     // settle: where each region is left and (finish) entered, which of them
-    // are, and the threads whose region is not settled; chase: where the chain
+    // are, and the threads whose region is not settled (in the batches: whose
+    // token is long); chase: where the chain
     // from a warp's position number `lane` leaves the warp's regions, where
     // lane 0's enters each of them, where the tile's chain enters the warp's
     // and leaves the tile
     uint32_t exit[kThreads], entry[kThreads];
     uint32_t entered[kWarps], votes[kWarps];
     uint32_t tile_exit;
-    int32_t event[kThreads];    // an event token's ladder status (OK: terminal)
+    int32_t event[kThreads];    // an event token's code
     uint32_t wsum[2][kWarps];   // scans: per-warp totals, used in turn
     Cut cut[2];                 // batches in turn
     uint64_t far;               // the successor past 2^31, see kExitFar
@@ -933,38 +948,114 @@ struct Chunk {
         }
     }
 
-    // One token longer than kBig (or with literals past the staged input) at
-    // input position P: copied by the whole CTA, its exact 64-bit lengths
-    // from the ladder, which has accepted it. Returns whether it is the
-    // chunk's last.
-    CDB_HD bool exec_big(uint64_t P) {
+    // A match of ml bytes at `to`, every byte before it written, by the whole
+    // CTA: in waves that never read their own output, or from its period.
+    CDB_HD void copy_match(uint8_t* to, uint64_t ml, uint64_t off) {
+        if (off >= 16 * kThreads || ml <= off) {
+            for (uint64_t k = 0; k < ml; k += off)
+                each([&](uint32_t t) {
+                    lzg::copy_share(to + k, to + k - off, ml - k < off ? ml - k : off, t,
+                                    kThreads);
+                });
+        } else {
+            const uint32_t f = static_cast<uint32_t>(off);
+            each([&](uint32_t t) {
+                for (uint32_t j = t; j < f; j += kThreads)
+                    s.u.e.period[j] = (to - off)[j];
+            });
+            each([&](uint32_t t) {
+                lzg::period_share(to, s.u.e.period, f, ml, t, kThreads);
+            });
+        }
+    }
+
+    // A long token of a batch (its first sector at base), output [r.out, end).
+    CDB_HD void exec_long(uint8_t* base, const Rec& r, uint32_t end) {
+        if (r.le != r.out)
+            each([&](uint32_t t) {
+                lzg::copy_share(base + r.out, s.in[buf] + (r.out + r.dl), r.le - r.out, t,
+                                kThreads);
+            });
+        if (end != r.le) copy_match(base + r.le, end - r.le, r.off);
+        LZC_PHASE(7);
+        LZC_EVENT(4, 1);
+    }
+
+    // The token at input position P, which the ladder has accepted: copied by
+    // the whole CTA, its exact 64-bit lengths from the ladder. Returns whether
+    // it is the chunk's last.
+    CDB_HD bool exec_far(uint64_t P) {
         lzl::Seq sq;
         (void)ladder_at(P, d, &sq);
         if (sq.lit)
             each([&](uint32_t t) {
                 lzg::copy_share(dst + d, g + sq.lit_src, sq.lit, t, kThreads);
             });
-        const uint64_t ms = d + sq.lit, ml = sq.ml, off = sq.off;
-        if (ml && off >= 16 * kThreads) {
-            // waves that never read their own output
-            for (uint64_t k = 0; k < ml; k += off)
-                each([&](uint32_t t) {
-                    lzg::copy_share(dst + ms + k, dst + ms + k - off, ml - k < off ? ml - k : off,
-                                    t, kThreads);
-                });
-        } else if (ml) {
-            const uint32_t f = static_cast<uint32_t>(off);
-            each([&](uint32_t t) {
-                for (uint32_t j = t; j < f; j += kThreads) s.u.period[j] = dst[ms - f + j];
-            });
-            each([&](uint32_t t) {
-                lzg::period_share(dst + ms, s.u.period, f, ml, t, kThreads);
-            });
-        }
-        d = ms + ml;
+        if (sq.ml) copy_match(dst + d + sq.lit, sq.ml, sq.off);
+        d += sq.lit + sq.ml;
         LZC_PHASE(7);
         LZC_EVENT(4, 1);
         return sq.done;
+    }
+
+    // Tokens [i, j) of a batch, none of them long, output [y, z) past base;
+    // `mapped`: the map holds them for the window at 0.
+    CDB_HD void gather(uint8_t* base, uint32_t i, uint32_t j, uint32_t y, uint32_t z,
+                       bool mapped) {
+        for (uint32_t W = mapped ? 0 : y & ~31u; W < z; W += kWindow) {
+            if (W || !mapped) {
+                each([&](uint32_t t) {
+                    for (uint32_t k = t; k < kSectors; k += kThreads) s.u.e.map[k].starts = 0;
+                });
+                each([&](uint32_t t) {
+                    if (t >= i && t < j)
+                        lzg::map_token(s.u.e.map, t, s.u.e.rec[t].out,
+                                       t + 1 < j ? s.u.e.rec[t + 1].out : z, W);
+                    if (t == i && W <= y) s.u.e.map[0].before = i;
+                });
+            }
+            copy_window(base, y, z, W);
+            LZC_EVENT(5, 1);
+        }
+    }
+
+    // The first long token of [i, m), or m.
+    CDB_HD uint32_t next_long(uint32_t i, uint32_t m) const {
+        for (; i < m; i = (i | 31) + 1) {
+            const uint32_t v = s.votes[i / 32] >> (i % 32);
+            if (v != 0) {
+                i += ctz64(v);
+                return i < m ? i : m;
+            }
+        }
+        return m;
+    }
+
+    // Tokens [0, m) of a batch, output up to y1, some of them long: the runs
+    // between those are gathered.
+    CDB_HD void exec_longs(uint8_t* base, uint32_t m, uint32_t y1) {
+        vote(s.votes, [&](uint32_t t) {
+            if (t >= m) return false;
+            const Rec r = s.u.e.rec[t];
+            return (t + 1 < m ? s.u.e.rec[t + 1].out : y1) - r.out > kBig || r.off >> 31;
+        });
+        for (uint32_t i = 0; i < m;) {
+            const uint32_t j = next_long(i, m);
+            const uint32_t y = s.u.e.rec[i].out, z = j < m ? s.u.e.rec[j].out : y1;
+            if (z > y) gather(base, i, j, y, z, i == 0);
+            LZC_PHASE(6);
+            if (j < m) exec_long(base, s.u.e.rec[j], j + 1 < m ? s.u.e.rec[j + 1].out : y1);
+            i = j + 1;
+        }
+    }
+
+    // The same out of line, so that it does not weigh on the registers and the
+    // code of batches without long tokens.
+    LZC_APART static void run_longs(Shm<F, kThreads>& s, uint32_t buf, uint8_t* base, uint32_t m,
+                                    uint32_t y1) {
+        Chunk c{s, nullptr, 0, nullptr, 0, 0};
+        c.buf = buf;
+        c.exec_longs(base, m, y1);
     }
 
     // Tokens [0, ntok) of the tile. Returns a status, and in *done whether
@@ -995,7 +1086,7 @@ struct Chunk {
                     fast[t] = true;
                     olen[t] = tok[t].lit + tok[t].ml;
                 } else {
-                    // clamped: a token longer than kBig ends the batch
+                    // clamped: such a token ends the batch
                     uint64_t ol = 0;
                     (void)F::step(reader(), S, e + p, &ol);
                     olen[t] = ol > 65536 ? 65536u : static_cast<uint32_t>(ol);
@@ -1011,62 +1102,50 @@ struct Chunk {
                 if (t >= n) return;
                 Tok& tk = tok[t];
                 uint32_t ls = tk.ls, off = tk.off, lit = tk.lit, ml = tk.ml;
-                bool big = false;
                 if (!fast[t] || !F::admit(tk, out[t], have, room)) {
                     lzl::Seq sq;
                     const uint64_t P = e + s.u.e.pos[b0 + t];
                     const int st = ladder_at(P, d + out[t], &sq);
                     uint64_t ol = 0;
                     const uint64_t nx = P < S ? F::step(reader(), S, P, &ol) : kStepEnd;
-                    bool event = st != CUDEC_OK || sq.done;
-                    s.event[t] = st;
-                    if (!event && nx != sq.next) {  // cannot happen: the steps are the ladder's
-                        s.event[t] = CUDEC_ERR_CUDA;
-                        event = true;
+                    const bool far =
+                        sq.lit > kBig || sq.ml > kBig ||
+                        (sq.lit && (sq.lit_src - e > lim || sq.lit > lim - (sq.lit_src - e)));
+                    if (st != CUDEC_OK || sq.done || far || nx != sq.next) {
+                        const bool lost = !sq.done && nx != sq.next;  // cannot happen: the steps
+                                                                      // are the ladder's
+                        s.event[t] = st != CUDEC_OK ? st : lost ? CUDEC_ERR_CUDA : far ? kFar : kEnd;
+                        at_min(&ct.event, t);
                     }
-                    if (event) at_min(&ct.event, t);
-                    big = sq.lit && (sq.lit_src - e > lim || sq.lit > lim - (sq.lit_src - e));
-                    big = big || sq.lit > kBig || sq.ml > kBig;
-                    lit = big ? 0 : static_cast<uint32_t>(sq.lit);
-                    ml = big ? 0 : static_cast<uint32_t>(sq.ml);
+                    lit = far ? 0 : static_cast<uint32_t>(sq.lit);
+                    ml = far ? 0 : static_cast<uint32_t>(sq.ml);
                     off = sq.off;
                     ls = static_cast<uint32_t>(sq.lit_src - e);
                 }
-                big = big || lit + ml > kBig || off >> 31;  // the gather's limits
                 const uint32_t y = y0 + out[t];
                 const uint32_t le = y + lit;
                 s.u.e.rec[t] = Rec{y, le, at0 + ls - y, off};
-                if (big) at_min(&ct.big, t);
-                else lzg::map_token(s.u.e.map, t, y, le + ml, 0);
+                if (lit + ml > kBig || off >> 31) {  // the gather's limits
+                    // (code for long ones costs Snappy batches without them 2 %)
+                    if (F::kSnappy) s.event[t] = kFar;
+                    at_min(F::kSnappy ? &ct.event : &ct.big, t);
+                } else lzg::map_token(s.u.e.map, t, y, le + ml, 0);
                 if (t == 0) s.u.e.map[0].before = 0;
             });
             const uint32_t ev = ct.event, bg = ct.big;
             LZC_PHASE(5);
             LZC_EVENT(3, 1);
-            // tokens [0, k) are gathered; then the event or the big token
-            uint32_t k = ev < bg ? ev : bg;
-            if (k > n) k = n;
-            const bool at_event = ev == k && k < n;
-            if (at_event && s.event[k] != CUDEC_OK) return s.event[k];
-            const bool last = at_event && bg != k;  // terminal, gathered with the batch
-            const uint32_t y1 = last     ? s.u.e.rec[k].le
-                                : k == 0 ? y0
-                                : k < n  ? s.u.e.rec[k].out
-                                         : y0 + total;
-            for (uint32_t W = 0; y1 > y0 && W < y1; W += kWindow) {
-                if (W) {
-                    each([&](uint32_t t) {
-                        for (uint32_t i = t; i < kSectors; i += kThreads) s.u.e.map[i].starts = 0;
-                    });
-                    each([&](uint32_t t) {
-                        if (t < k || (last && t == k)) {
-                            const uint32_t end = t + 1 < n ? s.u.e.rec[t + 1].out : y0 + total;
-                            lzg::map_token(s.u.e.map, t, s.u.e.rec[t].out, t == k ? y1 : end, W);
-                        }
-                    });
-                }
-                copy_window(base, y0, y1, W);
-                LZC_EVENT(5, 1);
+            // tokens [0, k), then the event
+            const uint32_t k = ev < n ? ev : n;
+            const int32_t code = k < n ? s.event[k] : kFar;
+            if (code != kEnd && code != kFar) return code;
+            const bool last = code == kEnd;
+            const uint32_t m = k + last;
+            const uint32_t y1 = last ? s.u.e.rec[k].le : k < n ? s.u.e.rec[k].out : y0 + total;
+            if (F::kSnappy || bg >= m) {
+                if (y1 > y0) gather(base, 0, m, y0, y1, true);
+            } else {
+                run_longs(s, buf, base, m, y1);
             }
             LZC_PHASE(6);
             d += y1 - y0;
@@ -1076,7 +1155,7 @@ struct Chunk {
             }
             if (k < n) {
                 const uint64_t P = e + s.u.e.pos[b0 + k];
-                if (exec_big(P)) {
+                if (exec_far(P)) {
                     *done = true;
                     return CUDEC_OK;
                 }

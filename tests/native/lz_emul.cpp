@@ -51,6 +51,9 @@ struct Caps {
 
 }  // namespace
 
+// Barriers that the CTA of the last run met.
+extern "C" uint32_t lz_barriers() { return emul::cta()->bars[0].gen; }
+
 // The large chunks of a batch, as the wide kernel's `wide` CTAs pick them
 // (chunk[0, *count): its index, one per CTA) and as the narrow CTAs of the m
 // chunks at `ask` find them (is[0, m)); reads: capacities that those m read.

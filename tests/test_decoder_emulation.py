@@ -21,6 +21,7 @@ import pytest
 
 import oracle
 from cudec_b200 import workload as W
+from lz_blocks import lz4_block, snappy_block
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -168,6 +169,58 @@ def test_lz(lz, size, threads):
             for m in range(4 if size < 6000 else 1):
                 check(lz(fmt, threads), want, mutate(rng, f), size - (m % 2) * size // 2,
                       starving(m, late) if m % 2 else m, 0, (size, k, fmt, m))
+
+
+def long_tokens(rng, n, share):
+    """Sequences of which `share` are longer than 1,024 bytes, by literals or by
+    a match from near or far; runs of the others longer than a window."""
+    seqs, total = [], 0
+    for _ in range(n):
+        lit, ml, off = rng.randbytes(rng.randrange(0, 40)), rng.randrange(4, 60), None
+        if rng.random() < share:
+            size = rng.choice([985, 1024, 1025, 1500, 4000])
+            if rng.random() < 0.3:
+                lit = rng.randbytes(size)
+            else:
+                ml = size
+        if not seqs:
+            lit = rng.randbytes(50)
+        total += len(lit)
+        off = rng.choice([1, 3, 31, 2000, 5000, 9000, 60000])
+        seqs.append((lit, min(off, total, 65535), ml))
+        total += ml
+    return seqs
+
+
+# Long tokens one after the other, at a batch's ends and between runs that fill
+# more than a window of output.
+@pytest.mark.parametrize("threads", [128, 512])
+@pytest.mark.parametrize("share", [0.02, 0.1, 1.0])
+def test_lz_long_tokens(lz, threads, share):
+    rng = random.Random(share)
+    for k in range(2):
+        n = (130, 600)[k] if share < 0.1 else 40
+        seqs = long_tokens(rng, n, share)
+        for fmt, pack, want in ((0, lz4_block, oracle.lz4_decode),
+                                (1, snappy_block, oracle.snappy_decode)):
+            comp = pack(seqs, rng.randbytes((20, 1500)[k]))
+            cap = sum(len(lit) + ml for lit, _, ml in seqs) + (20, 1500)[k]
+            assert want(comp, cap)[0] == 0
+            seed = starving(k, rng.randrange(threads // 32))
+            check(lz(fmt, threads), want, comp, cap, seed, (5 * k + fmt) % 16, (share, k, fmt))
+            check(lz(fmt, threads), want, mutate(rng, comp), cap, seed, 3, (share, k, fmt, "m"))
+
+
+def test_lz_long_tokens_share_a_batch(lz):
+    # literals and a match each cost a barrier; a batch of its own for every
+    # long token was two more
+    seqs = [(b"0123456789" * 200, 5000 if i > 5 else 7, 1500) for i in range(30)]
+    comp, cap = lz4_block(seqs, bytes(20)), 30 * 3500 + 20
+    check(lz(0, 512), oracle.lz4_decode, comp, cap, 1)
+    many = lz.lib.lz_barriers()
+    comp, cap = lz4_block(seqs[:10], bytes(20)), 10 * 3500 + 20
+    check(lz(0, 512), oracle.lz4_decode, comp, cap, 1)
+    assert many - lz.lib.lz_barriers() <= 20 * 2 + 40  # and the tiles of 40,000 bytes more
 
 
 def capacities(kind, n):
