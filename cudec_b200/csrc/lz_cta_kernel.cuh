@@ -119,6 +119,7 @@ constexpr uint32_t kExitMax = 0x80000000u;   // positions are below this
 
 // Step results (absolute positions otherwise).
 constexpr uint64_t kStepEnd = ~0ull;
+constexpr uint64_t kLenMax = 65536;  // a batch clamps longer tokens, which are its last
 constexpr uint32_t kSlowRel = 0xFFFFFFFFu;  // a fast step declines: the generic step decides
 constexpr uint32_t kStepSlow = 255;         // no short step from this position
 // Widest CTA whose regions are settled in rounds rather than chased. Us with
@@ -285,7 +286,8 @@ struct Lz4F : lzl::Lz4Ladder {
     static constexpr uint32_t kMinStep = 3;  // tokens with a successor span >= 3 bytes
     static constexpr bool kSnappy = false;
 
-    template <class R>
+    // kLen: only *olen is asked for, and above kLenMax only that it is.
+    template <bool kLen = false, class R>
     CDB_HD static uint64_t step(const R& in, uint64_t S, uint64_t P, uint64_t* olen) {
         if (P >= S) return kStepEnd;
         const uint32_t tok = in.at(P);
@@ -297,9 +299,10 @@ struct Lz4F : lzl::Lz4Ladder {
                 if (q >= S) return kStepEnd;
                 b = in.at(q++);
                 lit += b;
-            } while (b == 255);
+            } while (b == 255 && !(kLen && lit > kLenMax));
         }
         *olen = lit;
+        if (kLen && lit > kLenMax) return kStepEnd;
         if (lit > S - q || S - q - lit < kSrcSlack) return kStepEnd;
         q += lit + 2;
         uint64_t ml = (tok & 15) + 4;
@@ -308,7 +311,7 @@ struct Lz4F : lzl::Lz4Ladder {
                 if (q >= S) return kStepEnd;
                 b = in.at(q++);
                 ml += b;
-            } while (b == 255);
+            } while (b == 255 && !(kLen && ml > kLenMax));
         }
         *olen = lit + ml;
         return q;
@@ -420,7 +423,7 @@ struct SnappyF : lzl::SnappyLadder {
     static constexpr uint32_t kMinStep = 2;  // elements span >= 2 bytes
     static constexpr bool kSnappy = true;
 
-    template <class R>
+    template <bool kLen = false, class R>
     CDB_HD static uint64_t step(const R& in, uint64_t S, uint64_t P, uint64_t* olen) {
         if (P >= S) return kStepEnd;
         const uint32_t tag = in.at(P);
@@ -1088,8 +1091,8 @@ struct Chunk {
                 } else {
                     // clamped: such a token ends the batch
                     uint64_t ol = 0;
-                    (void)F::step(reader(), S, e + p, &ol);
-                    olen[t] = ol > 65536 ? 65536u : static_cast<uint32_t>(ol);
+                    (void)F::template step<true>(reader(), S, e + p, &ol);
+                    olen[t] = static_cast<uint32_t>(ol > kLenMax ? kLenMax : ol);
                 }
             });
             const uint32_t total = scan(olen, out);
@@ -1106,15 +1109,16 @@ struct Chunk {
                     lzl::Seq sq;
                     const uint64_t P = e + s.u.e.pos[b0 + t];
                     const int st = ladder_at(P, d + out[t], &sq);
-                    uint64_t ol = 0;
-                    const uint64_t nx = P < S ? F::step(reader(), S, P, &ol) : kStepEnd;
+                    // the chain's next token is the ladder's (or past the tile)
+                    const bool lost = b0 + t + 1 < ntok && e + s.u.e.pos[b0 + t + 1] != sq.next;
                     const bool far =
                         sq.lit > kBig || sq.ml > kBig ||
                         (sq.lit && (sq.lit_src - e > lim || sq.lit > lim - (sq.lit_src - e)));
-                    if (st != CUDEC_OK || sq.done || far || nx != sq.next) {
-                        const bool lost = !sq.done && nx != sq.next;  // cannot happen: the steps
-                                                                      // are the ladder's
-                        s.event[t] = st != CUDEC_OK ? st : lost ? CUDEC_ERR_CUDA : far ? kFar : kEnd;
+                    if (st != CUDEC_OK || sq.done || far || lost) {
+                        s.event[t] = st != CUDEC_OK          ? st
+                                     : lost && !sq.done ? CUDEC_ERR_CUDA  // cannot happen
+                                     : far              ? kFar
+                                                        : kEnd;
                         at_min(&ct.event, t);
                     }
                     lit = far ? 0 : static_cast<uint32_t>(sq.lit);

@@ -254,8 +254,14 @@ inline uint32_t __funnelshift_rc(uint32_t lo, uint32_t hi, uint32_t s) {
 inline uint32_t __funnelshift_lc(uint32_t lo, uint32_t hi, uint32_t s) {
     return s >= 32 ? lo : __funnelshift_l(lo, hi, s);
 }
+// Thread 0's loads through the read-only path.
+inline uint64_t& emul_ldgs() {
+    static uint64_t n = 0;
+    return n;
+}
 template <class T>
 T __ldg(const T* p) {
+    emul_ldgs() += emul::cta()->cur == 0;
     return *p;
 }
 

@@ -14,6 +14,7 @@ int run(const uint8_t* src, uint64_t S, uint8_t* dst, uint64_t cap, uint64_t see
     using Shm = cdb::lzc::Shm<F, T>;
     static Shm* shm = new Shm();
     std::memset(static_cast<void*>(shm), 0x5C, sizeof *shm);  // stale state must not matter
+    emul_ldgs() = 0;
     std::vector<int> st(T, -2);
     std::vector<uint64_t> out(T, 0);
     const bool ok = emul::run(T, seed, [&] {
@@ -51,8 +52,10 @@ struct Caps {
 
 }  // namespace
 
-// Barriers that the CTA of the last run met.
+// Barriers that the CTA of the last run met, and thread 0's loads of input past
+// the staged bytes.
 extern "C" uint32_t lz_barriers() { return emul::cta()->bars[0].gen; }
+extern "C" uint64_t lz_ldgs() { return emul_ldgs(); }
 
 // The large chunks of a batch, as the wide kernel's `wide` CTAs pick them
 // (chunk[0, *count): its index, one per CTA) and as the narrow CTAs of the m

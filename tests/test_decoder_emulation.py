@@ -49,6 +49,7 @@ def lz():
     lib.lz_emulate.argtypes = [ctypes.c_int, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_uint64,
                                ctypes.c_void_p, ctypes.c_uint64, ctypes.c_uint64,
                                ctypes.POINTER(ctypes.c_uint64)]
+    lib.lz_ldgs.restype = ctypes.c_uint64
     lib.lz_large.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_uint32, ctypes.c_uint64,
                              ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t,
                              ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)]
@@ -221,6 +222,14 @@ def test_lz_long_tokens_share_a_batch(lz):
     comp, cap = lz4_block(seqs[:10], bytes(20)), 10 * 3500 + 20
     check(lz(0, 512), oracle.lz4_decode, comp, cap, 1)
     assert many - lz.lib.lz_barriers() <= 20 * 2 + 40  # and the tiles of 40,000 bytes more
+
+
+def test_lz_passes_over_a_long_token(lz):
+    # 12,000 bytes of extension, some 4,800 of them past the staged input: walked
+    # on the chain, in the list, by the ladder and for the copy
+    comp = lz4_block([(b"abc", 3, 255 * 12000)], bytes(13))
+    check(lz(0, 128), oracle.lz4_decode, comp, 255 * 12000 + 16, 1)
+    assert lz.lib.lz_ldgs() < 4.5 * (12000 - 128 * 52 - 512)
 
 
 def capacities(kind, n):
