@@ -286,6 +286,18 @@ def test_zstd(zstd, size):
     check(zstd["one"], oracle.zstd_decode, f, size + 9, 3, 1, (size, "room"))
 
 
+# Literals and little else: streams that end anywhere in a window of five
+# symbols, and around the length from which eight lanes share one.
+def test_zstd_literals(zstd):
+    rng = random.Random(3)
+    for size in list(range(64, 96)) + list(range(1700, 1712)) + [5000, 5003, 20001]:
+        data = bytes(min(int(rng.expovariate(0.2)), 255) for _ in range(size))
+        f = W.zstd_compress(data, 1, 20, False)
+        check(zstd["one"], oracle.zstd_decode, f, size, size % 251, size % 16, size)
+        for k in range(2):
+            check(zstd["one"], oracle.zstd_decode, mutate(rng, f), size, k, 0, (size, k))
+
+
 def test_zstd_mutants(zstd):
     rng = random.Random(11)
     frames = [(W.zstd_compress(d, lv, 20, True), size) for size in (300, 4000, 140000)
