@@ -9,10 +9,10 @@ copy probability 0.5), each block compressed with liblz4
 LZ4_compress_default. The reference's corpora (Silesia, enwik8) are not
 available; these synthetic chunks stand in for them.
 
-A step is one cudec_lz4_decompress_batch launch over the whole batch with
+A step is one cudec_lz4_decompress_batch call over the whole batch with
 inputs resident in HBM. The working set (~100 MB) would fit in the 126 MB
 L2, so L2 is flushed (a 256 MiB memset) before every timed launch and only
-the launch itself is bracketed by CUDA events on its stream.
+the call's kernels are bracketed by CUDA events on its stream.
 
   value     decompressed bytes / mean launch time (whole job: all ranks)
   e2e       the same metric through the C ABI with host buffers:
@@ -200,6 +200,13 @@ def workload(n, fmt="lz4"):
     raws = [buf[int(o):int(o) + CHUNK] for o in offs]
     comp = W.lz4_compress if fmt == "lz4" else W.snappy_compress
     return raws, [comp(r) for r in raws]
+
+
+def lz_launches(n, sms):
+    """Kernels that one LZ4 or Snappy batch call of n chunks launches
+    (cudec_b200/csrc/batch.cu, launch_lz_cta): wide and narrow CTAs side by side
+    above 3 chunks per SM and up to 2^17, one width otherwise."""
+    return 2 if 3 * sms < n <= 1 << 17 else 1
 
 
 def peaks():
@@ -929,7 +936,8 @@ def main():
             **({"reference_gpu": ref_gpu} if ref_gpu else {}),
             **({"mixed": mixed_line} if mixed_line else {}),
             **({"serve": serve_line} if serve_line else {}),
-            "gpu_launches": 2 * args.steps,  # wide and narrow CTAs (more than 3 chunks per SM)
+            "gpu_launches": args.steps * lz_launches(
+                n, torch.cuda.get_device_properties(local).multi_processor_count),
             "clocks": clocks.summary(),
         }
         if world == 1 and args.cpu_seconds > 0:
