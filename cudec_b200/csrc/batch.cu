@@ -35,14 +35,18 @@ constexpr int kMaxDevices = 64;
 std::atomic<int> g_sm_count[kMaxDevices];
 
 // Chunks per SM up to which a batch's chunks get 512 or 256 threads each. Us
-// per batch of 64 KiB LZ4 chunks with 512 / 256 / 128 threads on 148 SMs: 148
-// chunks 174 / 201 / 300, 300 chunks 330 / 216 / 312, 440 chunks 387 / 234 /
-// 337, 592 chunks 527 / 393 / 357, 1,024 chunks 856 / 563 / 447; 16 chunks of
-// 4 MiB 9,550 / 11,720 / 15,980. (Taken before wide CTAs chased their chain and
-// the copy was shortened; the chosen widths now take 136, 217 for 440 chunks,
-// 333, 410 and 6,050.)
+// per batch of 64 KiB chunks with 512 / 256 / 128 threads on 148 SMs (128: with
+// the wide kernel beside, which finds nothing): LZ4 74 chunks 129 / 166 / 275,
+// 148 131 / 168 / 275, 200 221 / 191 / 284, 296 244 / 191 / 287, 370 326 / 214 /
+// 311, 444 347 / 214 / 311, 518 426 / 330 / 317, 592 453 / 363 / 331, 1,036 770 /
+// 521 / 412; Snappy 148 146 / 189 / 290, 296 265 / 209 / 315, 444 379 / 231 /
+// 327, 592 490 / 381 / 340; 16 LZ4 chunks of 4 MiB 5,706 / 7,993 / 8,186.
 constexpr size_t kWideMax = 1, kMediumMax = 3;
-constexpr uint32_t kWideThreads = 256;  // beside narrow CTAs
+// Threads of the wide CTAs beside narrow ones. 512 are quicker where the largest
+// chunk ends the batch (8,000 uneven Snappy chunks 2,869 us instead of 4,228,
+// 2,000 1,551 and 2,259, 30,000 uneven LZ4 chunks 3,610 and 3,698; 1,024 alike
+// 412 and 412), and not measured yet over other sizes.
+constexpr uint32_t kWideThreads = 256;
 // Up to here the wide CTAs read every capacity each (148 x 1 MiB out of L2), and
 // the narrow ones of large chunks some of them (is_large). 100,000 LZ4 pages of
 // 4 KiB take 3,610 us; with 1,000, 50,000 or all of them in slots of 256 KiB
@@ -61,8 +65,9 @@ int device_sm_count(int dev) {
     return v;
 }
 
-// The kernels' shared state exceeds 48 KB: opted into once per device, format
-// and width.
+// The kernels' shared state is 29 KB with 128 threads, 56 KB with 256 and 111 KB
+// with 512. Above 48 KB it is opted into, once per device, format and width (the
+// narrow one's opt-in changes nothing).
 template <class F, uint32_t T>
 cudaError_t prepare_cta(int dev) {
     static std::atomic<bool> ready[kMaxDevices];

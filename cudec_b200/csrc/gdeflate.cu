@@ -19,9 +19,11 @@ namespace gdf {
 constexpr uint32_t kWarps = 4;
 constexpr int kSmem = static_cast<int>(kWarps * sizeof(Tables));
 
-// Resident CTAs per SM that the registers are compiled for: 4,096 pages are
-// one wave of 7 (1,825 us; 6: 2,675, 5: 2,696), 24 pages take the same with
-// any (878, 874, 864).
+// Resident CTAs per SM that the registers are compiled for. Us with 7 / 6 / 5,
+// pages of 64 KiB: 24 (50,001 bytes) 887 / 881 / 872; 1,000 1,233 / 1,225 /
+// 1,219; 2,000 1,400 / 1,399 / 1,392; 4,096 (one wave of 7) 1,821 / 2,699 /
+// 2,703; 5,000 2,778 / 2,807 / 2,935; 6,000 2,971 / 3,086 / 3,891; 16,384
+// 7,066 / 7,624 / 8,451.
 constexpr int kCtasPerSm = 7;
 
 __global__ void __launch_bounds__(32 * kWarps, kCtasPerSm)

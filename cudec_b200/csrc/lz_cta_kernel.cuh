@@ -58,12 +58,14 @@
 //      its period, 100 chunks of 64 KiB of matches of 1,100 to 4,000 bytes took
 //      269 us, 16 of 4 MiB 12,816; now 119 and 4,443.
 //
-// What bounds it: instruction issue (77 % of the issue slots at seven CTAs per
-// SM; 290,000 warp instructions per 64 KiB chunk of 5,250 tokens, two thirds
-// of them in the copy). The decoder before this one computed chain exits by
-// the format's branching step, merged 16-byte pieces per token into a
-// shared-memory ring with atomics, and spent 568,000. 1,024 chunks of 64 KiB
-// on a B200: LZ4 0.943 -> 0.401 ms (167 GB/s out), Snappy 1.149 -> 0.430.
+// What bounds it: instruction issue and the waits between barriers (65 % of the
+// issue slots at seven CTAs per SM; 254,000 warp instructions per 64 KiB chunk
+// of 5,250 tokens; per issued instruction 2.2 warps wait out fixed latencies,
+// 1.8 at a barrier, 0.8 for global memory). The decoder before this one
+// computed chain exits by the format's branching step, merged 16-byte pieces
+// per token into a shared-memory ring with atomics, and spent 568,000. 1,024
+// chunks of 64 KiB on a B200: LZ4 0.943 -> 0.411 ms (163 GB/s out), Snappy
+// 1.149 -> 0.432.
 //
 // Every phase is per-thread code between CTA barriers, driven through an
 // executor: on the device each phase runs once per thread followed by
@@ -150,9 +152,8 @@ inline uint32_t ctz64(uint64_t v) { return static_cast<uint32_t>(__builtin_ctzll
 // Profiling builds (-DCDB_PHASE_TIMING) accumulate, from thread 0 of every
 // CTA, the SM cycles of each phase and event counts over a launch. Cycles:
 // 0 stage, 1 steps, 2 exits and entries, 3 list, 4 parse and scan, 5 check and map,
-// 6 copy, 7 whole-CTA tokens. Events: 0 tiles, 1 tokens, 2 settle rounds,
-// regions chased,
-// 3 batches, 4 whole-CTA tokens, 5 windows.
+// 6 copy, 7 whole-CTA tokens. Events: 0 tiles, 1 tokens, 2 settle rounds or
+// regions chased, 3 batches, 4 whole-CTA tokens, 5 windows.
 #if defined(CDB_PHASE_TIMING) && defined(__CUDACC__)
 __device__ unsigned long long lzc_cycles[16];
 __device__ unsigned long long lzc_events[16];

@@ -60,7 +60,9 @@ constexpr int kClasses = 3 * kSizeClasses;
 constexpr uint32_t kCtaWarps = CUDEC_MIXED_CTA_WARPS;
 // Resident CTAs per SM, at most, of the two CTA grids: they share the SMs with
 // each other and with the warp grid. The Zstd grid's limit is its kernel's own;
-// the LZ grid leaves room for the warp grid.
+// the LZ grid leaves room for the warp grid. 10,000 uneven chunks of all formats
+// with an LZ grid of 3, 4, 5 or 6 per SM, two inputs in two runs each: 8.27 to
+// 9.13 ms, 8.25 to 8.44, 8.21 to 8.46, 8.21 to 8.53.
 constexpr int kCtaPerSmMax = 5, kZstdPerSmMax = 4;
 constexpr uint32_t kCtaSmem = kMaxOf(static_cast<uint32_t>(sizeof(lzc::Shm<lzc::Lz4F>)),
                                      static_cast<uint32_t>(sizeof(lzc::Shm<lzc::SnappyF>)));
@@ -280,10 +282,11 @@ __global__ void __launch_bounds__(kThreads, 2) mixed_kernel(Args a) {
 }
 
 // Warps per LZ4 / Snappy chunk by bucket when the plan is created: one warp
-// below 16 KiB, a whole CTA from 16 KiB up (what the tuner picks on B200
-// over 100,000 uneven LZ4 + Snappy chunks, run after run: small chunks keep
-// the warp grid busy beside the CTA grid, and the CTA decoder's parallel
-// parse wins from 16 KiB up); a GDeflate page is one warp's.
+// below 16 KiB, a whole CTA from 16 KiB up; a GDeflate page is one warp's. This
+// is what the tuner picked for 100,000 uneven LZ4 and Snappy chunks with an
+// earlier CTA decoder. With the present one it picks a CTA in every bucket:
+// 27.4 ms for those chunks, 29.6 with this table, 22.5 by one plain call per
+// format (whose large chunks get wide CTAs, batch.cu).
 constexpr uint32_t kDefaultWpc[kBuckets] = {1, 1, kCtaWarps, kCtaWarps, kCtaWarps, kCtaWarps};
 
 struct Key {

@@ -20,11 +20,18 @@
 // With one warp doing all of this in turn a sequence cost about 490 cycles in
 // the state chain (every lane repeating the whole decode) and 356 in
 // execution; the chain alone is some 170 cycles with four frames on an SM, and
-// the rest hides behind it. What bounds a launch now: execution, by instruction
-// issue, where the SMs are full of frames; a frame's own state chain where
-// they are not. Measured, L2 flushed: 512 frames of 1 MiB at level 3 25,825 us
-// before, 7,741 now; 24 frames of one block 4,292 and 1,101; the mixed plan's
-// batch of uneven chunks of all formats 31,882 and 8,084.
+// the rest hides behind it. What bounds a launch now is latency: a frame takes
+// about as long alone as among four on its SM, execution waiting for the match
+// bytes of each part and for its barriers, then the state chain. With 256
+// frames of 1 MiB a quarter of the issue slots are used, and per issued
+// instruction 3.4 warps wait at a barrier and 1.4 for global memory. Measured,
+// L2 flushed: 512 frames of 1 MiB at level 3 25,825 us before, 7,683 now; six
+// of 128 KiB 4,250 and 850; the mixed plan's batch of uneven chunks of all
+// formats 31,882 and 8,240. Slower than before: many small frames of few long
+// sequences (4,096 frames of 16 KiB: matches of 200 to 900 bytes 213 and 279,
+// literal runs and copies of 300 to 3,000 200 and 265, nearly all literals
+// 1,118 and 1,245): four frames on an SM, not sixteen and more, to hide each
+// other's waits.
 //
 // The warps meet at named barriers, every arrival matched by a wait:
 //   kBarItem   warps 0, 2-5: item i is in its buffer (two buffers in turn,

@@ -1,8 +1,8 @@
 // Host emulation of the CTA-per-chunk LZ decoder (cudec_b200/csrc/
 // lz_cta_kernel.cuh): the kernel's phases run for every thread in turn, so
-// the CPU tests can check the decoder's algorithm (tiling, segment exits,
-// candidate and tile chases, counts, checks, grouped execution, whole-CTA
-// copies) against the oracle without a GPU. Test infrastructure only.
+// the CPU tests can check the decoder's algorithm (tiling, region exits and
+// entries, the token list, batches, the gathered output, whole-CTA copies)
+// against the oracle without a GPU. Test infrastructure only.
 #include <cstdint>
 #include <cstring>
 #include <memory>
