@@ -25,12 +25,12 @@
 // bytes of each part and for its barriers, then the state chain. With 256
 // frames of 1 MiB a quarter of the issue slots are used, and per issued
 // instruction 3.4 warps wait at a barrier and 1.4 for global memory. Measured,
-// L2 flushed: 512 frames of 1 MiB at level 3 25,825 us before, 7,683 now; six
+// L2 flushed: 512 frames of 1 MiB at level 3 25,825 us before, 7,565 now; six
 // of 128 KiB 4,250 and 850; the mixed plan's batch of uneven chunks of all
 // formats 31,882 and 8,240. Slower than before: many small frames of few long
 // sequences (4,096 frames of 16 KiB: matches of 200 to 900 bytes 213 and 279,
 // literal runs and copies of 300 to 3,000 200 and 265, nearly all literals
-// 1,118 and 1,245): four frames on an SM, not sixteen and more, to hide each
+// 1,118 and 1,223): four frames on an SM, not sixteen and more, to hide each
 // other's waits.
 //
 // The warps meet at named barriers, every arrival matched by a wait:

@@ -451,21 +451,22 @@ __device__ inline void huf_build(HufSmem& h, unsigned count, unsigned tl, uint32
 // Decode symbols from bit position *bp down while it is above `end` and fewer
 // than `most` have been decoded; returns their number. put(i, symbol) takes
 // each, note(i, bp) each position before its symbol. Five symbols per window
-// (5 x 11 <= 55 bits, 11 the largest table log), without a test per symbol
-// while all five are wanted whatever their lengths: one warp of a frame's CTA
-// decodes its literals, so frames of little else wait for this loop. 4,096
-// frames of 16 KiB that are nearly all literals 1,279 us with the tests, 1,244
-// without; 96 of 260,000 bytes at level 19 1,776 and 1,594; 8,000 of 8,000
-// bytes 1,445 and 1,339; where execution is what frames wait for, 512 of 1 MiB
-// 7,671 and 7,683, 2,048 of them 26,889 and 27,139.
-template <class Put, class Note>
+// (5 x 11 <= 55 bits, 11 the largest table log). kWhole: without a test per
+// symbol while all five are wanted whatever their lengths. One warp of a frame's
+// CTA decodes its literals, so frames of little else wait for these loops. Us
+// with the tests everywhere; without them in the eight lanes' first pass and
+// for a lane alone; in their writing pass too: 4,096 frames of 16 KiB that are
+// nearly all literals 1,282, 1,223, 1,246; 96 of 260,000 bytes at level 19
+// 1,774, 1,590, 1,591; 8,000 of 8,000 bytes 1,450, 1,349, 1,339; 512 of 1 MiB
+// 7,683, 7,565, 7,719; 2,048 of them 26,916, 26,769, 27,248.
+template <bool kWhole, class Put, class Note>
 __device__ __forceinline__ uint32_t huf_run(const BitWin& bw, const uint16_t* cells, unsigned tl,
                                             int32_t* bp, int32_t end, uint32_t most, Put put,
                                             Note note) {
     uint32_t n = 0;
     int32_t p = *bp;
     // windows whose five symbols are all wanted, whatever their lengths
-    while (p - end > 5 * 11 && most - n >= 5) {
+    while (kWhole && p - end > 5 * 11 && most - n >= 5) {
         uint32_t hi, lo;
         bw.window(p, &hi, &lo);
         uint32_t at = 0;
@@ -549,11 +550,12 @@ __device__ inline bool huf_streams(const uint8_t* pay, uint64_t psize, unsigned 
         const int32_t from = T - static_cast<int32_t>(j) * part;
         const int32_t end = j + 1 == per ? 0 : from - part;
         int32_t x = from;
-        const uint32_t n1 = huf_run(bw, h.cells, tl, &x, end, ~0u, no_put,
-                                    [&](uint32_t i, int32_t p) {
-                                        if (i < kMergeMax)
-                                            h.merge[i][lane] = static_cast<uint16_t>(from - p);
-                                    });
+        const uint32_t n1 = huf_run<true>(bw, h.cells, tl, &x, end, ~0u, no_put,
+                                          [&](uint32_t i, int32_t p) {
+                                              if (i < kMergeMax)
+                                                  h.merge[i][lane] =
+                                                      static_cast<uint16_t>(from - p);
+                                          });
         // the true start, and the symbols up to the first noted position
         int32_t start = __shfl_up_sync(0xffffffffu, x, 1);
         if (j == 0) start = T;
@@ -569,7 +571,7 @@ __device__ inline bool huf_streams(const uint8_t* pay, uint64_t psize, unsigned 
                 }
                 gp = from - h.merge[g][lane];
             } else {
-                nt += huf_run(bw, h.cells, tl, &p, p - 1, 1, no_put, no_note);
+                nt += huf_run<false>(bw, h.cells, tl, &p, p - 1, 1, no_put, no_note);
             }
         }
         split = __all_sync(0xffffffffu, merged);
@@ -584,9 +586,9 @@ __device__ inline bool huf_streams(const uint8_t* pay, uint64_t psize, unsigned 
             const bool ok = j + 1 != per || (x == 0 && incl == n_want);
             if (!__all_sync(0xffffffffu, ok)) return false;
             uint8_t* o = out + (incl - n);
-            (void)huf_run(bw, h.cells, tl, &start, -(1 << 30), n,
-                          [&](uint32_t i, uint32_t sym) { o[i] = static_cast<uint8_t>(sym); },
-                          no_note);
+            (void)huf_run<false>(
+                bw, h.cells, tl, &start, -(1 << 30), n,
+                [&](uint32_t i, uint32_t sym) { o[i] = static_cast<uint8_t>(sym); }, no_note);
             __syncwarp();
             return true;
         }
@@ -594,9 +596,9 @@ __device__ inline bool huf_streams(const uint8_t* pay, uint64_t psize, unsigned 
     bool ok = true;
     if (j == 0) {
         int32_t p = T;
-        (void)huf_run(bw, h.cells, tl, &p, -(1 << 30), n_want,
-                      [&](uint32_t i, uint32_t sym) { out[i] = static_cast<uint8_t>(sym); },
-                      no_note);
+        (void)huf_run<true>(
+            bw, h.cells, tl, &p, -(1 << 30), n_want,
+            [&](uint32_t i, uint32_t sym) { out[i] = static_cast<uint8_t>(sym); }, no_note);
         ok = p == 0;
     }
     ok = __all_sync(0xffffffffu, ok);
